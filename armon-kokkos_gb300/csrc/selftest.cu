@@ -201,8 +201,8 @@ __global__ void mul_check(uint64_t seed, int64_t n, unsigned long long* out)
     }
 }
 
-// The division's quotient estimate against exact 128-bit arithmetic: the remainder
-// ma 2^52 - q mb must lie in [0, 2 mb) (one correction step then gives the quotient).
+// The division's quotient estimate against exact 128-bit arithmetic, for dividends in [mb, 2 mb): the
+// remainder ma 2^52 - q mb must be the one returned and lie in [0, 1.5 mb).
 __global__ void quot_check(uint64_t seed, int64_t n, unsigned long long* out)
 {
     using namespace armon::sfp;
@@ -211,14 +211,15 @@ __global__ void quot_check(uint64_t seed, int64_t n, unsigned long long* out)
         uint64_t mb = (r2 & kMant) | kHidden;
         if ((r3 & 15) == 0) mb = kHidden + 1;                       // just above a power of two
         if ((r3 & 15) == 1) mb = (kHidden << 1) - 1;                // just below the next
-        if (mb == kHidden) mb += 1;
+        if ((r3 & 15) == 2) mb = kHidden;
         uint64_t ma = (r1 & kMant) | kHidden;
-        if ((r3 >> 4) & 1) ma <<= 1;                                // the doubled dividend
-        if ((r3 & 0xE0) == 0x20) ma = (r3 >> 8) & 1 ? (kHidden << 2) - 1 : kHidden;
-        const uint64_t q = quot_estimate(ma, recip_v(mb));
+        if ((r3 & 0xE0) == 0x20) ma = (r3 >> 8) & 1 ? mb : mb - 1;   // the ends of the range
+        if (ma < mb) ma <<= 1;                                      // the doubled dividend
+        uint64_t r;
+        const uint64_t q = quot_estimate(ma, mb, recip_y(mb), r);
         const unsigned __int128 num = (unsigned __int128)ma << 52;
         const unsigned __int128 qm = (unsigned __int128)q * mb;
-        const bool ok = qm <= num && num - qm < 2 * (unsigned __int128)mb;
+        const bool ok = qm <= num && num - qm == r && 2 * r < 3 * mb;
         if (!ok && atomicAdd(&out[0], 1ull) == 0) {
             out[2] = ma;
             out[3] = mb;

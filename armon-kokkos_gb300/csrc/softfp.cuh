@@ -16,17 +16,14 @@
 //   mul(a, b)     the correctly rounded product
 //   add(a, b)     the correctly rounded sum (add_bits: the same on bit patterns, host or device)
 //
-// Division (my own construction from the arithmetic, not a library's sequence).  With
-// significands ma, mb in [2^52, 2^53) and ma doubled when ma < mb, the result significand is
-// Q = floor(ma * 2^52 / mb) rounded with the remainder R = ma * 2^52 - Q * mb.  Q is estimated
-// with a reciprocal of d = mb * 2^11: an FP32 seed (rcp.approx of the top 24 bits), biased below
-// the true value, then two Newton steps y <- y + y (1 - d y) in 64-bit fixed point, each of which
-// keeps the estimate below 2^128 / d; then Q_est = floor(U * V / 2^128) for U = ma * 2^63.  The
-// remainder is computed exactly in 64 bits and Q_est is raised once if R >= mb.  If R still is not
-// in [0, mb) -- which the error bounds exclude -- the hardware division is used, so a fast-path
-// result always satisfies ma * 2^52 = Q * mb + R with 0 <= R < mb, i.e. Q is exact.  Zero
-// dividends are handled; subnormal, infinite and NaN operands and quotients outside the normal
-// range go to the hardware division.
+// Division (my own construction from the arithmetic, not a library's sequence).  With significands
+// ma, mb in [2^52, 2^53) and ma doubled when ma < mb, the result significand is ma 2^52 / mb rounded to
+// nearest.  A 32-bit reciprocal of mb (an FP32 seed and one Newton step in 32-bit fixed point, from
+// below) gives the quotient in two digits, each followed by its exact remainder, and the last
+// remainder decides the rounding: see quot_estimate for the bounds.  32-bit products only, about 60
+// instructions with the exponent handling (two Newton steps in 64-bit fixed point and a correction
+// step took about 100).  Zero dividends are handled; subnormal, infinite and NaN operands and
+// quotients outside the normal range go to the hardware division.
 #pragma once
 
 #include <cstdint>
@@ -111,48 +108,49 @@ __device__ __forceinline__ double scale(double x, int k, double p2)
 __device__ __forceinline__ double half(double x) { return scale(x, -1, 0.5); }
 __device__ __forceinline__ double twice(double x) { return scale(x, 1, 2.0); }
 
-// The reciprocal of a divisor significand mb in (2^52, 2^53): V = 2^64 + v ~ 2^128 / d for
-// d = mb 2^11, from below.
-__device__ __forceinline__ uint64_t recip_v(uint64_t mb)
+// A 32-bit reciprocal of a divisor significand mb in [2^52, 2^53): y <= 2^84 / mb < 2^32, within 2^-30
+// of it (relative).  The seed is rcp.approx (one ulp) of mb's top 24 bits, made odd so that it stays
+// above 2^23 and its reciprocal below 2^-23; with 1/x for x = mb / 2^53 in units of 2^-31, the
+// truncation (2^9), the odd bit (2^9) and the seed's ulp (2^8) leave it within [-0x300, 0x300] of
+// the true value, so that less 0x400 it lies in [-0x700, -0x100].  One Newton step y += y (1 - x y)
+// in 32 bits, with x rounded up, keeps it below and leaves 2^-40 (the step), 2^-31 (x) and 2^-31 (the
+// truncation).
+__host__ __device__ __forceinline__ uint32_t mulhi32(uint32_t a, uint32_t b)
 {
-    const uint64_t d = mb << 11;                                   // [2^63, 2^64)
-    const uint32_t top = (uint32_t)(d >> 40);                      // [2^23, 2^24)
-    const float fd = __uint_as_float(0x4B000000u | (top & 0x7FFFFFu));   // == top
+    return (uint32_t)(((uint64_t)a * b) >> 32);
+}
+__host__ __device__ __forceinline__ uint32_t recip_step(uint32_t dhi, uint32_t seed_bits)
+{
+    const uint32_t y0 = ((seed_bits << 8) | 0x80000000u) - 0x400u;
+    const uint64_t e = (1ull << 63) - ((uint64_t)dhi * y0 + y0);        // 1 - x y0 in Q63, below 2^43
+    return y0 + (mulhi32(y0, (uint32_t)(e >> 11)) >> 20);
+}
+__device__ __forceinline__ uint32_t recip_y(uint64_t mb)
+{
+    const uint32_t dhi = (uint32_t)(mb >> 21);
+    const float fd = __uint_as_float(0x4B000001u | ((dhi >> 8) & 0x7FFFFFu));
     float rf;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rf) : "f"(fd));
-    const uint32_t urf = __float_as_uint(rf);
-    // rf in (2^-24, 2^-23]; rf * 2^88 = 2^64 (1 + m 2^-23) when rf < 2^-23.  The seed is lowered
-    // by 2^44 (2^-21 relative) so that it is below 2^128 / d.
-    uint64_t v;
-    if ((urf >> 23) >= 104u) {
-        v = 0xFFFFF00000000000ull;
-    } else {
-        const uint64_t m = (uint64_t)(urf & 0x7FFFFFu) << 41;
-        v = m > (1ull << 44) ? m - (1ull << 44) : 0;
-    }
-#pragma unroll
-    for (int it = 0; it < 2; it++) {
-        // e = 2^128 - d (2^64 + v) >= 0; its high word, then V += V e / 2^128 (from below)
-        const uint64_t ph = __umul64hi(d, v);
-        const uint64_t pl = d * v;
-        const uint64_t eh = 0ull - d - ph - (pl != 0 ? 1ull : 0ull);
-        v = v + eh + __umul64hi(v, eh);
-    }
-    return v;
+    return recip_step(dhi, __float_as_uint(rf));
 }
 
-// The quotient estimate of significands ma in [2^52, 2^54) and mb (reciprocal V = 2^64 + v):
-// floor(x (2^64 + v) / 2^74) for x = ma 2^9 (< 2^63).  V lies within 2^-62 below 2^128 / d, so the
-// estimate is floor(ma 2^52 / mb) or one less.
-__device__ __forceinline__ uint64_t quot_estimate(uint64_t ma, uint64_t v)
+// The quotient ma 2^52 / mb of significands ma in [mb, 2 mb) from mb's reciprocal y, in two digits of
+// 27 and 26 bits: q1 falls short of ma 2^26 / mb by less than 1.25 (half a quarter each for ma's and
+// y's truncation, one for the floor), so r1 = ma 2^26 - q1 mb < 1.25 mb; q2 of r1 2^26 / mb by less
+// than 1.14 in the same way.  The result q is then floor(ma 2^52 / mb) or one less, and r = ma 2^52 -
+// q mb, exact in 64 bits, lies in [0, 1.14 mb).
+__host__ __device__ __forceinline__ uint64_t quot_estimate(uint64_t ma, uint64_t mb, uint32_t y, uint64_t& r)
 {
-    const uint64_t x = ma << 9;
-    return (x + __umul64hi(x, v)) >> 10;
+    const uint32_t q1 = mulhi32((uint32_t)(ma >> 22), y) >> 4;
+    const uint64_t r1 = (ma << 26) - (uint64_t)q1 * mb;
+    const uint32_t q2 = mulhi32((uint32_t)(r1 >> 22), y) >> 4;
+    r = (r1 << 26) - (uint64_t)q2 * mb;
+    return ((uint64_t)q1 << 26) + q2;
 }
 
-// a / b; the reciprocal comes from get_v(mb), called only on the integer path.
-template <class GetV>
-__device__ __forceinline__ double div_core(double a, double b, uint64_t ub, GetV get_v)
+// a / b; the reciprocal comes from get_y(mb), called only on the integer path.
+template <class GetY>
+__device__ __forceinline__ double div_core(double a, double b, uint64_t ub, GetY get_y)
 {
     const uint64_t ua = bits(a);
     const uint32_t ea = (uint32_t)(ua >> 52) & 0x7FFu;
@@ -160,90 +158,71 @@ __device__ __forceinline__ double div_core(double a, double b, uint64_t ub, GetV
     const uint64_t sign = (ua ^ ub) & ~kAbs;
     const int e0 = (int)ea - (int)eb;
     const bool b_normal = (eb - 1u) < 2046u;
-    if (b_normal && (ua << 1) == 0) return from_bits(sign);   // +-0 / normal
-    if (!(b_normal && (ea - 1u) < 2046u && e0 >= -1021 && e0 <= 1022)) return a / b;
-
+    if (!(b_normal && (ea - 1u) < 2046u && (unsigned)(e0 + 1021) <= 2043u)) {
+        if (b_normal && (ua << 1) == 0) return from_bits(sign);   // +-0 / normal
+        return a / b;
+    }
     uint64_t ma = (ua & kMant) | kHidden;
     const uint64_t mb = (ub & kMant) | kHidden;
-    int e = e0;
-    if (ma < mb) {
-        ma <<= 1;
-        e -= 1;
-    }
-    uint64_t q;
+    const uint32_t less = ma < mb ? 1u : 0u;
+    ma <<= less;
     uint64_t r;
-    if (mb == kHidden) {
-        // a power-of-two divisor: the quotient is the dividend's significand, exactly
-        q = ma;
-        r = 0;
-    } else {
-        // Q_est is Q or Q - 1, and one correction step makes it Q
-        q = quot_estimate(ma, get_v(mb));
-        r = (ma << 52) - q * mb;          // exact: the true remainder lies in [0, 2 mb)
-        const bool up1 = r >= mb;
-        r = up1 ? r - mb : r;
-        q = up1 ? q + 1 : q;
-        if (r >= mb) return a / b;        // outside the error bounds: the hardware decides
-    }
-    // round to nearest, ties to even, on the exact remainder
-    const uint64_t r2 = r << 1;
-    const bool up = r2 > mb || (r2 == mb && (q & 1));
-    q += up ? 1ull : 0ull;
-    return from_bits(sign + ((uint64_t)(e + 1022) << 52) + q);
+    uint64_t q = quot_estimate(ma, mb, get_y(mb), r);
+    // Round to nearest.  A quotient of doubles is never halfway between two doubles, so with
+    // r in [0, 1.14 mb) the rounded significand is q + 1 when 2 r > mb and q otherwise: for r >= mb
+    // the quotient is q + 1 and what is left of r is below half of mb.
+    q += (r << 1) > mb ? 1ull : 0ull;
+    return from_bits(sign + ((uint64_t)(uint32_t)(e0 + 1022 - (int)less) << 52) + q);
 }
 
 __device__ __forceinline__ double div(double a, double b)
 {
-    return div_core(a, b, bits(b), [](uint64_t mb) { return recip_v(mb); });
+    return div_core(a, b, bits(b), [](uint64_t mb) { return recip_y(mb); });
 }
 
-// A divisor's reciprocal computed once for several quotients (when it is not a power of two and
-// the divisor is normal; div(a, R, b) is exact whatever R holds for other divisors).
+// A divisor's reciprocal computed once for several quotients (of a normal divisor; div(a, R, b) is
+// exact whatever R holds for other divisors).
 struct Recip {
-    uint64_t ub, v;
+    uint64_t ub;
+    uint32_t y;
 };
 
 __device__ __forceinline__ Recip recip(double b)
 {
     Recip R;
     R.ub = bits(b);
-    const uint64_t mb = (R.ub & kMant) | kHidden;
-    const uint32_t eb = (uint32_t)(R.ub >> 52) & 0x7FFu;
-    R.v = (mb != kHidden && (eb - 1u) < 2046u) ? recip_v(mb) : 0;
+    R.y = recip_y((R.ub & kMant) | kHidden);
     return R;
 }
 
 __device__ __forceinline__ double div(double a, const Recip& R, double b)
 {
-    return div_core(a, b, R.ub, [&](uint64_t) { return R.v; });
+    return div_core(a, b, R.ub, [&](uint64_t) { return R.y; });
 }
 
 // Multiplication (my own construction).  For normal operands with significands ma, mb in
-// [2^52, 2^53) the exact product ma mb lies in [2^104, 2^106); with both significands shifted to
-// bit 63, the high word of their 128-bit product holds its top 64 bits and the low word the rest.
-// The top 53 bits are the result significand, the next bit the rounding bit and everything below
-// it the sticky part; round to nearest, ties to even.  Zero operands give signed zeros; subnormal,
-// infinite and NaN operands and results outside the normal range take the FP64 multiply.
+// [2^52, 2^53), both shifted to bit 63, the product lies in [2^126, 2^128); shifted to bit 127, its
+// high word holds the result significand over 11 bits of rest, the lowest of which also stands for
+// everything below (a sticky bit); round to nearest, ties to even.  Zero operands give signed zeros;
+// subnormal, infinite and NaN operands and results near or outside the ends of the normal range
+// take the FP64 multiply.
 __device__ __forceinline__ double mul(double a, double b)
 {
     const uint64_t ua = bits(a), ub = bits(b);
     const uint32_t ea = (uint32_t)(ua >> 52) & 0x7FFu;
     const uint32_t eb = (uint32_t)(ub >> 52) & 0x7FFu;
     const uint64_t sign = (ua ^ ub) & ~kAbs;
-    if ((ea - 1u) < 2046u && (eb - 1u) < 2046u) {
-        const uint64_t xa = ((ua & kMant) | kHidden) << 11;      // [2^63, 2^64)
+    const uint32_t e = ea + eb - 1024u;      // the result's biased exponent less one, before normalisation
+    if ((ea - 1u) < 2046u && (eb - 1u) < 2046u && e < 2044u) {
+        const uint64_t xa = ((ua & kMant) | kHidden) << 11;
         const uint64_t xb = ((ub & kMant) | kHidden) << 11;
-        const uint64_t hi = __umul64hi(xa, xb);                  // [2^62, 2^64)
-        const bool lo_nz = xa * xb != 0;
-        const uint32_t top = (uint32_t)(hi >> 63);               // product >= 2^105
-        const uint32_t sh = 10 + top;
-        const uint64_t m = hi >> sh;                             // [2^52, 2^53)
-        const uint64_t rem = hi & ((1ull << sh) - 1);
-        const uint64_t halfw = 1ull << (sh - 1);
-        const bool up = rem > halfw || (rem == halfw && (lo_nz || (m & 1)));
-        const int e = (int)ea + (int)eb - 1023 + (int)top;      // biased exponent of the result
-        if ((unsigned)(e - 1) < 2046u) return from_bits(sign + ((uint64_t)(e - 1) << 52) + m + (up ? 1u : 0u));
-        return a * b;
+        const unsigned __int128 p = (unsigned __int128)xa * xb;
+        const uint64_t hi = (uint64_t)(p >> 64), lo = (uint64_t)p;
+        const uint32_t top = (uint32_t)(hi >> 63);
+        const uint64_t w = (top ? hi : (hi << 1) | (lo >> 63)) | (lo != 0 ? 1u : 0u);
+        const uint64_t m = w >> 11;
+        const uint32_t up = ((uint32_t)w & 0x7FFu) + ((uint32_t)m & 1u) > 0x400u ? 1u : 0u;
+        return from_bits(sign + ((uint64_t)(e + top) << 52) + m + up);
     }
     if (((ua << 1) == 0 && (eb - 1u) < 2046u) || ((ub << 1) == 0 && (ea - 1u) < 2046u) ||
         ((ua << 1) == 0 && (ub << 1) == 0))
