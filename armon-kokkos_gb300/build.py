@@ -33,6 +33,7 @@ UNITS = [
     ("sweep_f64.cu", ["--fmad=false"]),
     ("sweep_f32.cu", ["--fmad=false"]),
     ("sweep_split.cu", ["--fmad=false"]),
+    ("sweep_tile.cu", ["--fmad=false"]),
     ("abi_kernels.cu", ["--fmad=false"]),
     ("solver.cu", ["--fmad=false"]),
     ("batch.cu", ["--fmad=false"]),

@@ -31,7 +31,16 @@ struct StepState {
     int32_t cycle, status;
     uint32_t counter;               // block-completion counter of the dt reduction
     int32_t buf_base;               // state buffer set = (cycle * passes + pass + buf_base) % 2
+    uint64_t max_x, max_y;          // tile passes: bit patterns of the dt maxima so far in this cycle
 };
+
+// Counters of a tile launch, shared by its blocks; the last block to finish leaves them zero.
+struct TileCtl {
+    uint32_t ticket, arrived;
+};
+
+// Tiles of a large unit (sweep_tile.cuh).
+constexpr int kTileUnit = 8;
 
 enum : int32_t { STATUS_RUNNING = 0, STATUS_INVALID_DT = 1 };
 

@@ -36,6 +36,14 @@ int sweep_batch_split_blocks_per_sm(bool fp32, int scheme, int proj, int block);
 // Blocks of the split pass's cell half (sweep_cells_kernel, last pass of a cycle) resident on one SM.
 int sweep_split_blocks_per_sm(bool fp32, int scheme, int proj, int block);
 
+// Tile axis pass (sweep_tile.cuh): `grid` resident blocks; ctl starts as zeros and is left so.
+cudaError_t launch_sweep_tile(const SweepArgs<double>& a, TileCtl* ctl, int scheme, int proj, bool last, int grid,
+                              cudaStream_t st);
+cudaError_t launch_sweep_tile(const SweepArgs<float>& a, TileCtl* ctl, int scheme, int proj, bool last, int grid,
+                              cudaStream_t st);
+// Blocks of the tile pass resident on one SM.
+int sweep_tile_blocks_per_sm(bool fp32, int scheme, int proj);
+
 // Fused axis pass over many domains (sweep_batch_kernel): doms / offsets are device arrays.
 cudaError_t launch_sweep_batch(const SweepArgs<double>* doms, const int* offsets, int ndom, int total_blocks, int pass,
                                BatchOrder ord, int scheme, int proj, bool last, int block, cudaStream_t st);

@@ -37,7 +37,8 @@ struct armon_solver {
     size_t elem = 8;
     void* arr[16] = {};
     bool owns_arrays = false;
-    StepState* d_state = nullptr;
+    StepState* d_state = nullptr;   // followed by the tile launches' counters
+    TileCtl* d_ctl = nullptr;
     StepState* h_state = nullptr;   // pinned
     double* d_partials = nullptr;
     double* d_cons = nullptr;       // conservation partials + 2 results
@@ -76,6 +77,10 @@ struct armon_solver {
     int order_cap = 0;
     bool split = false;             // each pass as a face launch and a cell launch (sweep_split.cuh)
     bool default_split = false;     // the form before any measurement
+    bool tile = false;              // each pass in the tile form (sweep_tile.cuh)
+    bool default_tile = false;
+    int tile_lines = 0;             // columns of a Y tile (0: the default)
+    int tile_per_sm = 0;            // blocks of the tile kernel resident on an SM
     void* d_faces = nullptr;        // 3 * face_stride values
     int64_t face_stride = 0;
 };
@@ -94,6 +99,8 @@ int cuda_fail(cudaError_t e, const char* what)
         if (e_ != cudaSuccess) return cuda_fail(e_, #expr);       \
     } while (0)
 
+constexpr int kTileYLines = 4;
+
 template <class T>
 void fill_geom(armon_solver* s, SweepArgs<T>& a)
 {
@@ -110,6 +117,17 @@ void fill_geom(armon_solver* s, SweepArgs<T>& a)
     if (s->split) {
         a.faces = static_cast<T*>(s->d_faces);
         a.face_stride = s->face_stride;
+    }
+    if (s->tile) {
+        if (s->tile_per_sm == 0) s->tile_per_sm = sweep_tile_blocks_per_sm(s->fp32, s->p.scheme, s->p.projection);
+        const int slots = s->sm_count * s->tile_per_sm;
+        int units = 1;
+        for (int axis = 0; axis < 2; axis++) {
+            set_tile_axis(a.geom[axis], axis == 0, stencil_reach(&s->p), s->sm_count, slots,
+                          s->tile_lines > 0 ? s->tile_lines : kTileYLines);
+            units = std::max(units, a.geom[axis].tile_units);
+        }
+        s->grid = std::min(slots, units);
     }
 }
 
@@ -133,7 +151,7 @@ int order_arrays_held(const armon_solver* s) { return s->d_faces ? 4 : 2; }
 // The next passes' unit order from the costs the last passes recorded.
 int launch_order(armon_solver* s)
 {
-    if (!s->ordered) return ARMON_OK;
+    if (!s->ordered || s->tile) return ARMON_OK;
     UnitCounts n{{axis_blocks(s, 0), axis_blocks(s, 1), axis_blocks(s, 0), axis_blocks(s, 1)}};
     order_units_kernel<<<order_arrays(s), 1024, 0, s->stream>>>(s->d_cost, s->d_order, s->order_cap, n);
     CUDA_TRY(cudaGetLastError());
@@ -145,7 +163,7 @@ int launch_order(armon_solver* s)
 // and starts from index order.
 int prepare_order(armon_solver* s)
 {
-    if (!s->ordered) return ARMON_OK;
+    if (!s->ordered || s->tile) return ARMON_OK;
     const int need = std::max(axis_blocks(s, 0), axis_blocks(s, 1));
     if (need > s->order_cap) {
         CUDA_TRY(cudaStreamSynchronize(s->stream));
@@ -184,6 +202,11 @@ int prepare_order(armon_solver* s)
 
 cudaError_t launch_pass(armon_solver* s, int k, bool last)
 {
+    if (s->tile) {
+        s->a32.pass = s->a64.pass = k;
+        return s->fp32 ? launch_sweep_tile(s->a32, s->d_ctl, s->p.scheme, s->p.projection, last, s->grid, s->stream)
+                       : launch_sweep_tile(s->a64, s->d_ctl, s->p.scheme, s->p.projection, last, s->grid, s->stream);
+    }
     if (s->fp32) {
         s->a32.pass = k;
         return s->split ? launch_sweep_split(s->a32, s->p.scheme, s->p.projection, last, s->grid, s->block, s->stream)
@@ -237,7 +260,7 @@ int enqueue_steady(armon_solver* s, int n_cycles)
         if (rc != ARMON_OK) return rc;
         while (n_cycles >= s->graph_cycles) {
             CUDA_TRY(cudaGraphLaunch(s->graph, s->stream));
-            s->launches += (int64_t)s->graph_cycles * (s->npass * (s->split ? 2 : 1) + (s->ordered ? 1 : 0));
+            s->launches += (int64_t)s->graph_cycles * (s->npass * (s->split ? 2 : 1) + (s->ordered && !s->tile ? 1 : 0));
             n_cycles -= s->graph_cycles;
         }
     }
@@ -286,7 +309,10 @@ int ensure_stage(armon_solver* s)
 // the best, a few cycles' worth.  A loop that ends before the measurement does keeps the model's
 // tiling and caches nothing.  Domains under 2^20 cells, single-pass splittings and a caller-fixed
 // seg_len are left to the model.
-using Tiling = std::array<int, 4>;   // segment length X, segment length Y, block lines, split form
+// segment length X, segment length Y, block lines, form (0 fused, 1 split); or for tiles (form
+// kTileForm): 0, columns of a Y tile, block lines, form
+using Tiling = std::array<int, 4>;
+constexpr int kTileForm = 2;
 std::map<std::array<int, 9>, Tiling> g_tilings;
 std::mutex g_tilings_mu;
 constexpr int kTuneDelay = 16;
@@ -319,7 +345,9 @@ int apply_tiling(armon_solver* s, const Tiling& t)
     s->tuned_seg[0] = t[0];
     s->tuned_seg[1] = t[1];
     s->block = t[2];
-    s->split = t[3] != 0 && s->d_faces != nullptr;
+    s->tile = t[3] == kTileForm;
+    if (s->tile) s->tile_lines = t[1];
+    s->split = t[3] == 1 && s->d_faces != nullptr;
     int rc = refill(s);
     return rc != ARMON_OK ? rc : ensure_partials(s);
 }
@@ -334,7 +362,7 @@ std::array<int, 9> tiling_key(const armon_solver* s)
 // the cost model's tiling in the solver's default form
 Tiling model_tiling(const armon_solver* s)
 {
-    return Tiling{0, 0, s->o.block_lines > 0 ? s->o.block_lines : 128, s->default_split ? 1 : 0};
+    return Tiling{0, 0, s->o.block_lines > 0 ? s->o.block_lines : 128, s->default_tile ? kTileForm : s->default_split ? 1 : 0};
 }
 
 void end_tuning(armon_solver* s)
@@ -364,8 +392,10 @@ int start_tuning(armon_solver* s)
     const int halo = stencil_reach(&p);
     const int block = s->o.block_lines > 0 ? s->o.block_lines : 128;
     std::vector<int> forms;
-    if (s->d_faces && s->o.split_pass == 0) forms = {1, 0}; else forms = {s->split ? 1 : 0};
     auto& T = s->tune;
+    if (s->tile) {
+        for (int lines : {4, 8, 2}) T.cand.push_back(Tiling{0, lines, block, kTileForm});
+    } else if (s->d_faces && s->o.split_pass == 0) forms = {1, 0}; else forms = {s->split ? 1 : 0};
     for (int form : forms) {
         const int per_sm = form ? sweep_split_blocks_per_sm(s->fp32, p.scheme, p.projection, block)
                                 : sweep_blocks_per_sm(s->fp32, p.scheme, p.projection, block);
@@ -574,7 +604,9 @@ static int solver_create(const armon_params* p, const armon_solver_opts* opts, d
     s->elem = s->fp32 ? 4 : 8;
     s->block = s->o.block_lines > 0 ? s->o.block_lines : 128;
     s->ordered = s->o.unit_order >= 0;
-    s->split = s->o.split_pass > 0 || (s->o.split_pass == 0 && !s->fp32);
+    // the tile form unless the caller asks for something of the marches'
+    s->tile = s->default_tile = s->o.split_pass == 0 && s->o.seg_len <= 0 && s->o.block_lines <= 0;
+    s->split = !s->tile && (s->o.split_pass > 0 || (s->o.split_pass == 0 && !s->fp32));
     if (s->block % 32 != 0 || s->block > 128) { delete s; set_error("block_lines must be a multiple of 32, at most 128"); return ARMON_ERR_PARAMS; }
     s->graph_cycles = s->o.cycles_per_graph;
     s->npass = passes_per_cycle(p->axis_splitting);
@@ -607,7 +639,8 @@ static int solver_create(const armon_params* p, const armon_solver_opts* opts, d
             }
         }
     }
-    e = cudaMalloc(&s->d_state, sizeof(StepState));
+    e = cudaMalloc(&s->d_state, sizeof(StepState) + sizeof(TileCtl));
+    s->d_ctl = reinterpret_cast<TileCtl*>(s->d_state + 1);
     if (e == cudaSuccess) e = cudaMallocHost(&s->h_state, sizeof(StepState));
     // the partial buffers are sized after the geometry is known
     s->cfg = make_step_config(*p);
@@ -630,7 +663,7 @@ static int solver_create(const armon_params* p, const armon_solver_opts* opts, d
         }
     }
     s->default_split = s->split;
-    if (e == cudaSuccess) e = cudaMemsetAsync(s->d_state, 0, sizeof(StepState), s->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(s->d_state, 0, sizeof(StepState) + sizeof(TileCtl), s->stream);
     if (e != cudaSuccess) { armon_solver_destroy(s); return cuda_fail(e, "solver allocation"); }
     std::memset(s->h_state, 0, sizeof(StepState));
     if (s->fp32) fill_geom(s, s->a32); else fill_geom(s, s->a64);
@@ -877,8 +910,12 @@ int64_t armon_solver_kernel_launches(armon_solver* s) { return s->launches; }
 int armon_solver_tiling(armon_solver* s, int32_t seg_len[2], int32_t blocks[2])
 {
     for (int axis = 0; axis < 2; axis++) {
-        const int sl = s->fp32 ? s->a32.geom[axis].seg_len : s->a64.geom[axis].seg_len;
-        const int nb = s->fp32 ? s->a32.geom[axis].blocks : s->a64.geom[axis].blocks;
+        const auto pick = [&](const auto& g, int& sl, int& nb) {
+            sl = s->tile ? g.tile_len : g.seg_len;
+            nb = s->tile ? std::min(s->grid, g.tile_units) : g.blocks;
+        };
+        int sl, nb;
+        if (s->fp32) pick(s->a32.geom[axis], sl, nb); else pick(s->a64.geom[axis], sl, nb);
         if (seg_len) seg_len[axis] = sl;
         if (blocks) blocks[axis] = nb;
     }

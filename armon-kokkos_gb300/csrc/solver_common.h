@@ -73,6 +73,39 @@ inline AxisTiling choose_segments(int n, int nlines, int block, int halo, int sm
     return axis_tiling(n, nlines, block, best_seg);
 }
 
+// Threads of a tile (sweep_tile.cuh).
+constexpr int kTileBlock = 256;
+
+// The tiles of one axis.  A tile is `lines` lines by width = len + 2 halo positions, at most kTileBlock
+// threads.  Along rows (X) the positions are consecutive in memory, so a tile is as long as the block
+// allows; along columns (Y) the lines are, so a tile takes y_lines of them and what length is left.
+// The segments of a line are made equal.  A domain with fewer tiles than SMs takes fewer lines per
+// tile: a pass over it lasts as long as one position's chain, whatever a tile holds.  Large units
+// leave about four tiles per resident block to single-tile units, which end the launch evenly.
+template <class T>
+void set_tile_axis(AxisGeom<T>& g, bool rows, int halo, int sms, int slots, int y_lines)
+{
+    const int want = rows ? 1 : std::max(1, std::min(y_lines, g.nlines));
+    const int longest = std::max(1, std::min(248, kTileBlock / want - 2 * halo));
+    int segs = (g.n + longest - 1) / longest;
+    const int len = (g.n + segs - 1) / segs;
+    segs = (g.n + len - 1) / len;
+    g.tile_len = len;
+    g.tile_width = len + 2 * halo;
+    g.tile_segs = segs;
+    const int fit = std::max(1, kTileBlock / g.tile_width);
+    const int spread = (int)std::max<int64_t>(1, (int64_t)g.nlines * segs / sms);
+    g.tile_lines = std::max(1, std::min({rows ? fit : std::min(fit, want), g.nlines, spread}));
+    g.tile_groups = (g.nlines + g.tile_lines - 1) / g.tile_lines;
+    g.tile_scan = rows ? g.tile_lines == 1 : g.tile_lines * kTileUnit <= 32 && len <= 56;
+    if (!rows && g.tile_scan)       // a large unit of columns lies in one segment
+        g.tile_groups = (g.tile_groups + kTileUnit - 1) / kTileUnit * kTileUnit;
+    const int64_t tiles = (int64_t)segs * g.tile_groups;
+    int64_t big = std::max<int64_t>(0, (tiles - 4 * (int64_t)slots) / kTileUnit);
+    g.tile_big = (int)big;
+    g.tile_units = (int)(big + (tiles - big * kTileUnit));
+}
+
 inline int check_supported(const armon_params* p)
 {
     if (!armon_params_check(p)) { set_error("invalid parameters (Params::check)"); return ARMON_ERR_PARAMS; }
@@ -161,6 +194,8 @@ int make_sweep_args(const armon_params& p, int npass, int block, int sms, const 
         g.cost = nullptr;
         g.face_order = nullptr;
         g.face_cost = nullptr;
+        g.tile_len = g.tile_width = g.tile_lines = g.tile_segs = g.tile_groups = g.tile_units = 0;
+        g.tile_big = g.tile_scan = 0;
     }
     a.origin = (int64_t)p.nb_ghosts * p.row_length + p.nb_ghosts;
     a.sw = p.stencil_width;

@@ -191,6 +191,15 @@ struct AxisGeom {
     uint32_t* cost;
     const uint32_t* face_order;   // the same for the face half of a split pass (sweep_split.cuh)
     uint32_t* face_cost;
+    // The tile form (sweep_tile.cuh): tiles of tile_lines lines by tile_len owned positions.
+    int32_t tile_len;     // owned positions of a tile
+    int32_t tile_width;   // tile_len plus the halo of both sides
+    int32_t tile_lines;   // lines of a tile
+    int32_t tile_segs;    // tiles along a line
+    int32_t tile_groups;  // tiles across the lines
+    int32_t tile_units;   // units of the axis: tile_big of kTileUnit consecutive tiles, then one tile each
+    int32_t tile_big;
+    int32_t tile_scan;    // units may be scanned for kept states (one row, or up to 32 columns, per unit)
 };
 
 template <class T>
@@ -470,51 +479,60 @@ __device__ __forceinline__ bool quotient_positive(double num, double den)
     return (int64_t)un > 0 && (unsigned)(en - 1) < 2046u && quotient_finite(num, den) && ed - en < 1000;
 }
 
+// The second-order advection flux of a face from its upwind side: Wl and u0 are the width and the
+// advected quantities of the upwind cell o, dm = L(o) - L(o-1), dp = L(o+1) - L(o), sm = W(o-1) + W(o),
+// sp = W(o) + W(o+1), Dx the face's length (src/kernels/euler_projection.cpp:82-120).
+template <class T>
+__device__ __forceinline__ Adv<T> advect2_upwind(T disp, T Dx, T Wl, const Adv<T>& u0, const Adv<T>& dm,
+                                                 const Adv<T>& dp, T sm, T sp)
+{
+    const T two_Dx_l = qtwice(Wl);
+    if constexpr (sizeof(T) == 8) {
+        // every slope a signed zero: the three quotients are not needed (exactly the same result)
+        if (ARMON_SOFT_FP64 && slope_is_zero(dm.r, dp.r) && slope_is_zero(dm.ra, dp.ra) &&
+            slope_is_zero(dm.ro, dp.ro) && slope_is_zero(dm.rE, dp.rE) &&
+            quotient_positive(two_Dx_l, sm) && quotient_positive(two_Dx_l, sp) && quotient_finite(Dx, two_Dx_l)) {
+            const uint64_t sx = sfp::bits(Dx) >> 63;
+            const auto prod = [&](T d_p) { return sfp::from_bits(((sfp::bits(d_p) >> 63) ^ sx) << 63); };
+            Adv<T> a;
+            a.r = qmul<6>(disp, u0.r - prod(dp.r));
+            a.ra = qmul<6>(disp, u0.ra - prod(dp.ra));
+            a.ro = qmul<6>(disp, u0.ro - prod(dp.ro));
+            a.rE = qmul<6>(disp, u0.rE - prod(dp.rE));
+            return a;
+        }
+    }
+    const T r_m = qdiv_at<6>(two_Dx_l, sm);          // 2 Dx_l / (Dx_l + Dx_lm)
+    const T r_p = qdiv_at<6>(two_Dx_l, sp);          // 2 Dx_l / (Dx_l + Dx_lp)
+    const T slope_r = slope_minmod(dm.r, dp.r, r_m, r_p);
+    const T slope_ra = slope_minmod(dm.ra, dp.ra, r_m, r_p);
+    const T slope_ro = slope_minmod(dm.ro, dp.ro, r_m, r_p);
+    const T slope_rE = slope_minmod(dm.rE, dp.rE, r_m, r_p);
+    const T length_factor = qdiv_at<7>(Dx, two_Dx_l);
+    Adv<T> a;
+    a.r = qmul<6>(disp, u0.r - qmul<6>(slope_r, length_factor));
+    a.ra = qmul<6>(disp, u0.ra - qmul<6>(slope_ra, length_factor));
+    a.ro = qmul<6>(disp, u0.ro - qmul<6>(slope_ro, length_factor));
+    a.rE = qmul<6>(disp, u0.rE - qmul<6>(slope_rE, length_factor));
+    return a;
+}
+
 template <class T>
 __device__ __forceinline__ Adv<T> advect2(const Flux<T>& Fm, const Flux<T>& Fk, const Flux<T>& Fp,
                                           const Lag<T>& L1, const Lag<T>& L2, const Adv<T>& d01,
                                           const Adv<T>& d12, const Adv<T>& d23, T s01, T s12, T s23, T dx)
 {
-    // src/kernels/euler_projection.cpp:82-120 for face k, from cells L1 = k-1 and L2 = k and the
-    // differences d01 = L(k-1) - L(k-2), d12 = L(k) - L(k-1), d23 = L(k+1) - L(k), and the width
-    // sums s01 = W(k-2) + W(k-1), s12, s23, which neighbouring faces share.  Upwind (disp > 0) the
-    // cells are (k-2, k-1, k), else (k-1, k, k+1).  x + y == y + x exactly, and
-    // -(dx - y) == -(dx + (-y)), so the face's Dx costs one addition.
-    T disp = Fk.dtus;
-    bool up = qgt0(disp);
-    T Dx = qneg_if(dx + (up ? qneg_if(Fm.dtus, true) : Fp.dtus), up);
-    const T Dx_l = up ? L1.W : L2.W;
-    const T two_Dx_l = qtwice(Dx_l);
-    if constexpr (sizeof(T) == 8) {
-        // every slope a signed zero: the three quotients are not needed (exactly the same result)
-        const Adv<T> dm = up ? d01 : d12, dp = up ? d12 : d23;
-        if (ARMON_SOFT_FP64 && slope_is_zero(dm.r, dp.r) && slope_is_zero(dm.ra, dp.ra) &&
-            slope_is_zero(dm.ro, dp.ro) && slope_is_zero(dm.rE, dp.rE) &&
-            quotient_positive(two_Dx_l, up ? s01 : s12) && quotient_positive(two_Dx_l, up ? s12 : s23) &&
-            quotient_finite(Dx, two_Dx_l)) {
-            const uint64_t sx = sfp::bits(Dx) >> 63;
-            const auto prod = [&](T d_p) { return sfp::from_bits(((sfp::bits(d_p) >> 63) ^ sx) << 63); };
-            Adv<T> a;
-            a.r = qmul<6>(disp, (up ? L1.rho : L2.rho) - prod(dp.r));
-            a.ra = qmul<6>(disp, (up ? L1.rua : L2.rua) - prod(dp.ra));
-            a.ro = qmul<6>(disp, (up ? L1.ruo : L2.ruo) - prod(dp.ro));
-            a.rE = qmul<6>(disp, (up ? L1.rE : L2.rE) - prod(dp.rE));
-            return a;
-        }
-    }
-    T r_m = qdiv_at<6>(two_Dx_l, up ? s01 : s12);    // 2 Dx_l / (Dx_l + Dx_lm)
-    T r_p = qdiv_at<6>(two_Dx_l, up ? s12 : s23);    // 2 Dx_l / (Dx_l + Dx_lp)
-    T slope_r = slope_minmod(up ? d01.r : d12.r, up ? d12.r : d23.r, r_m, r_p);
-    T slope_ra = slope_minmod(up ? d01.ra : d12.ra, up ? d12.ra : d23.ra, r_m, r_p);
-    T slope_ro = slope_minmod(up ? d01.ro : d12.ro, up ? d12.ro : d23.ro, r_m, r_p);
-    T slope_rE = slope_minmod(up ? d01.rE : d12.rE, up ? d12.rE : d23.rE, r_m, r_p);
-    T length_factor = qdiv_at<7>(Dx, two_Dx_l);
-    Adv<T> a;
-    a.r = qmul<6>(disp, (up ? L1.rho : L2.rho) - qmul<6>(slope_r, length_factor));
-    a.ra = qmul<6>(disp, (up ? L1.rua : L2.rua) - qmul<6>(slope_ra, length_factor));
-    a.ro = qmul<6>(disp, (up ? L1.ruo : L2.ruo) - qmul<6>(slope_ro, length_factor));
-    a.rE = qmul<6>(disp, (up ? L1.rE : L2.rE) - qmul<6>(slope_rE, length_factor));
-    return a;
+    // face k, from cells L1 = k-1 and L2 = k and the differences d01 = L(k-1) - L(k-2),
+    // d12 = L(k) - L(k-1), d23 = L(k+1) - L(k), and the width sums s01 = W(k-2) + W(k-1), s12, s23,
+    // which neighbouring faces share.  Upwind (disp > 0) the cells are (k-2, k-1, k), else
+    // (k-1, k, k+1).  x + y == y + x exactly, and -(dx - y) == -(dx + (-y)), so the face's Dx costs
+    // one addition.
+    const T disp = Fk.dtus;
+    const bool up = qgt0(disp);
+    const T Dx = qneg_if(dx + (up ? qneg_if(Fm.dtus, true) : Fp.dtus), up);
+    const Adv<T> u0{up ? L1.rho : L2.rho, up ? L1.rua : L2.rua, up ? L1.ruo : L2.ruo, up ? L1.rE : L2.rE};
+    return advect2_upwind(disp, Dx, up ? L1.W : L2.W, u0, up ? d01 : d12, up ? d12 : d23, up ? s01 : s12,
+                          up ? s12 : s23);
 }
 
 template <class T>

@@ -1,0 +1,824 @@
+// sweep_tile.cuh -- the axis pass with one thread per position: a block takes a tile (a few lines by a
+// stretch of positions, halo included), every thread computes each stage at its own position, and
+// the stages hand their values to the neighbouring positions through shared memory.
+//
+// Same stage functions on the same operands as the marches (sweep.cuh, sweep_split.cuh), so the
+// results are the same bits.
+//
+// Why tiles.  A march owns a segment of a line per thread: its positions run one after the other
+// (~1600 dependent instructions each), its pipeline keeps ~75 FP64 values alive (250 registers, 8
+// warps per SM), and in the X pass its warp loads touch 32 rows.  A tile's thread keeps one position,
+// and only a stage's operands are alive at once, so more warps share an SM, a pass over a small
+// domain lasts as long as one position's chain, and both axes read consecutive addresses.
+//
+// Tile geometry.  X pass: a tile is tile_lines rows by tile_width positions, thread = row * tile_width +
+// position, so a warp reads a stretch of a row.  Y pass: tile_lines columns by tile_width positions,
+// thread = position * tile_lines + column; the neighbours along the axis are tile_lines threads away.
+// tile_width = tile_len + 2 H positions (H = the stencil reach, 4 for GAD + second order), of which
+// the inner tile_len are stored.
+//
+// Units and dispatch.  Blocks stay resident; a block takes units of consecutive tiles, the first by its
+// index and the following ones from a ticket counter, so that tiles that cost more (fronts) spread
+// over the blocks by themselves.  The first tile_big units hold kTileUnit tiles, the rest one each,
+// so that the launch ends evenly.
+//
+// Exact reuse (SweepArgs::reuse).  A position whose window (H positions on either side) holds equal
+// cells, bit for bit, has results that depend on that cell's state alone.  A block keeps two such
+// states with their results, recorded by the thread at the middle of a computed stretch when its
+// window is uniform.  Once it keeps one it scans a unit before computing: every cell is loaded (the
+// loads of a batch issued together) and compared with the kept states, eight-position chunks whose
+// windows all hold a kept state get its results, and what is left becomes stretches (a line's
+// consecutive chunks) in a list.  The block computes the list packed, several stretches side by side
+// in its threads, so that a thin front costs its own positions and not whole tiles.  A unit without
+// a uniform chunk is computed as tiles, and a block that keeps no state does not scan.
+#pragma once
+
+#include "sweep.cuh"
+
+namespace armon {
+
+constexpr int kTileThreads = 256;
+constexpr int kTileWarps = kTileThreads / 32;
+constexpr int kTileSlots = 15;
+constexpr int kTileList = 512;        // stretches the list can hold (at most 128 per scan, 16 left over)
+
+#ifndef ARMON_TILE_MIN_BLOCKS
+#define ARMON_TILE_MIN_BLOCKS 3
+#endif
+#ifndef ARMON_TILE_MIN_BLOCKS_F32
+#define ARMON_TILE_MIN_BLOCKS_F32 4
+#endif
+template <class T> constexpr int tile_min_blocks() { return sizeof(T) == 8 ? ARMON_TILE_MIN_BLOCKS : ARMON_TILE_MIN_BLOCKS_F32; }
+
+// A kept state: the cell, its p and c, and the results of a position inside a run of it.
+enum : int { kRunRho, kRunUa, kRunUo, kRunE, kRunP, kRunC, kRunOut, kRunValues = kRunOut + 4 };
+
+// Consecutive owned positions of a line waiting to be computed.
+struct Stretch {
+    int32_t line;
+    int32_t start_len;    // first position << 8 | positions (at most 248)
+};
+
+template <class T>
+struct TileShared {
+    // Slots between the stages (a barrier after each stage's writes; a slot is only rewritten after a
+    // barrier that follows its last reads, the next tile's stages included):
+    //   cell products      rc, rcu, p, ua, dm                9-13
+    //   face differences   au, bu, ap, bp                    5-8
+    //   fluxes             u*, p*, p* u*, dt u*              0-3
+    //   Lagrangian cells   rho, rho ua, rho uo, rho E, W     4-8
+    //   their differences  four, and the width sum           9-13
+    //   advection fluxes   four                              0, 1, 2, 14
+    T ex[kTileSlots][kTileThreads];
+    T c[kTileThreads];                // sound speed of the position, for dt_CFL
+    T kept[2][kRunValues];
+    DtAcc acc[kTileThreads];
+    Stretch list[kTileList];          // a ring: entries head .. tail - 1
+    uint32_t match[2][2][kTileWarps][kTileWarps];   // [unit parity][kept state]: see scan_rows / scan_columns
+    uint32_t head;
+    uint32_t tail[2];                 // [unit parity]
+    int uniform[2];                   // [unit parity]: the unit holds a uniform chunk
+    int valid[2];
+    int turn;                         // the kept state to replace next
+    int next[2];                      // [unit parity]: the block's next unit
+};
+
+// The tiles of one unit of one domain.
+template <class T, int SCHEME, int PROJ>
+struct TilePass {
+    static constexpr bool kGAD = SCHEME == 1;
+    static constexpr bool kE2 = PROJ == 2;
+    static constexpr int H = 2 + (kGAD ? 1 : 0) + (kE2 ? 1 : 0);
+    static constexpr int kLagLo = kGAD ? 2 : 1;      // first position with a Lagrangian cell
+
+    const SweepArgs<T>& A;
+    TileShared<T>& sh;
+    int axis = 0, src = 0;
+    T dt{};
+    bool last = false, pcg = false;
+    int tile_q = 0, tile_l = 0;       // the thread's position and line in a tile
+    int parity = 0;
+
+    struct Spot {                     // the thread's place
+        int q, t, width;              // position in the stretch (halo included), along the axis; positions of the stretch
+        int64_t base;                 // index of position 0 of the line
+        bool in;
+    };
+
+    __device__ __forceinline__ TilePass(const SweepArgs<T>& a, TileShared<T>& s) : A(a), sh(s) {}
+
+    // Reads the domain's step state; false when this pass has nothing to do.
+    __device__ __forceinline__ bool start(int pass, bool last_pass, bool reports)
+    {
+        const StepState st = *A.state;
+        const CycleDt cd = cycle_time_step(st, A.cfg);
+        if (!cd.run) return false;
+        if (cd.invalid) {
+            if (last_pass && reports) A.state->status = STATUS_INVALID_DT;
+            return false;
+        }
+        double factor;
+        split_axis(A.cfg.splitting, st.cycle, pass, &axis, &factor);
+        dt = T(cd.current * factor);
+        src = (int)(((int64_t)st.cycle * A.npass + pass + st.buf_base) & 1);
+        last = last_pass;
+        pcg = A.write_eos > 0 || (last_pass && A.write_eos == 0);
+        const AxisGeom<T>& g = A.geom[axis];
+        const int tid = threadIdx.x;
+        if (axis == 0) {
+            tile_l = tid / g.tile_width;
+            tile_q = tid - tile_l * g.tile_width;
+        } else {
+            tile_q = tid / g.tile_lines;
+            tile_l = tid - tile_q * g.tile_lines;
+        }
+        return true;
+    }
+
+    // Segment and line group of a tile: along rows (X) consecutive tiles follow the line, along
+    // columns (Y) they lie side by side.
+    __device__ __forceinline__ void place(const AxisGeom<T>& g, int tile, int& seg, int& grp) const
+    {
+        if (axis == 0) { grp = tile / g.tile_segs; seg = tile - grp * g.tile_segs; }
+        else { seg = tile / g.tile_groups; grp = tile - seg * g.tile_groups; }
+    }
+    __device__ __forceinline__ Spot tile_spot(const AxisGeom<T>& g, int tile) const
+    {
+        int seg, grp;
+        place(g, tile, seg, grp);
+        const int a0 = seg * g.tile_len;
+        Spot p;
+        p.q = tile_q;
+        p.width = min(g.n, a0 + g.tile_len) - a0 + 2 * H;
+        p.t = a0 - H + tile_q;
+        const int line = grp * g.tile_lines + tile_l;
+        p.in = tile_q < p.width && tile_l < g.tile_lines && line < g.nlines;
+        p.base = A.origin + (int64_t)line * g.lstride;
+        return p;
+    }
+    // position t -> the cell read there: itself (real, or an untouched ghost past the mirrored band:
+    // stale), or the mirror of a real cell (side 1: low, 2: high); the same rule as the marches'
+    __device__ __forceinline__ bool source(int n, int t, int& m, int& side) const
+    {
+        m = t;
+        side = 0;
+        if (t < 0) {
+            if (t < -A.sw) return true;
+            m = -1 - t;
+            side = 1;
+        } else if (t >= n) {
+            if (t >= n + A.sw) return true;
+            m = 2 * n - 1 - t;
+            side = 2;
+        }
+        return false;
+    }
+    __device__ __forceinline__ void mirror(const AxisGeom<T>& g, CellIn<T>& c, int side) const
+    {
+        if (side) {
+            if (g.f_unit) {
+                const uint32_t b = side == 1 ? 0 : 2;
+                c.ua = qneg_if(c.ua, (g.fneg >> b) & 1u);
+                c.uo = qneg_if(c.uo, (g.fneg >> (b + 1)) & 1u);
+            } else {
+                c.ua = c.ua * (side == 1 ? g.fa_lo : g.fa_hi);
+                c.uo = c.uo * (side == 1 ? g.fo_lo : g.fo_hi);
+            }
+        }
+    }
+    __device__ __forceinline__ void load(int64_t i, CellIn<T>& c) const
+    {
+        T* const* in = A.buf[src];
+        c.rho = in[0][i];
+        c.ua = in[1 + axis][i];
+        c.uo = in[2 - axis][i];
+        c.E = in[3][i];
+    }
+    __device__ __forceinline__ bool same_as_kept(const CellIn<T>& c, int e) const
+    {
+        const T* k = sh.kept[e];
+        return same_bits(c.rho, k[kRunRho]) & same_bits(c.ua, k[kRunUa]) & same_bits(c.uo, k[kRunUo]) &
+               same_bits(c.E, k[kRunE]);
+    }
+
+    // The unit's tiles.  `after`, run by thread 0, gives the block's next unit, which is returned;
+    // when there is none (>= total), what the list still holds is computed too.
+    template <class After>
+    __device__ __forceinline__ int unit(int u, int total, After after)
+    {
+        const AxisGeom<T>& g = A.geom[axis];
+        int tile = u < g.tile_big ? u * kTileUnit : g.tile_big * kTileUnit + (u - g.tile_big);
+        const int end = u < g.tile_big ? tile + kTileUnit : tile + 1;
+        int next = total;
+        bool fetch = true;
+        while (tile < end) {
+            parity ^= 1;
+            if (threadIdx.x == 0) {
+                if (fetch) sh.next[parity] = after();
+                sh.tail[parity] = sh.tail[parity ^ 1];
+            }
+            const bool v0 = sh.valid[0] != 0, v1 = sh.valid[1] != 0;
+            // the same for every thread: a barrier follows each of their writes
+            const bool scan = g.tile_scan && (v0 || v1);
+            // a block that keeps no state yet takes a tile at a time, to scan the rest once it does
+            const int nk = scan || !g.tile_scan ? end - tile : 1;
+            int k = 0;
+            if (scan) {
+                if (axis == 0) scan_rows(g, tile, nk, v0, v1);
+                else scan_columns(g, tile, nk, v0, v1);
+                __syncthreads();
+                if (sh.uniform[parity]) {
+                    k = nk;
+                    if (axis == 0) fill_rows(g, tile, nk);
+                    else fill_columns(g, tile, nk);
+                }
+            }
+            __syncthreads();
+            if (threadIdx.x == 0) sh.uniform[parity ^ 1] = 0;    // for the next scan
+            if (fetch) next = sh.next[parity];
+            fetch = false;
+            const bool all = next >= total && tile + nk >= end;
+            // the tiles, or the list's stretches, packed
+            for (;;) {
+                Spot p;
+                int ds = 1, centre;
+                if (k < nk) {
+                    p = tile_spot(g, tile + k);
+                    if (axis != 0) ds = g.tile_lines;
+                    centre = (p.width / 2) * ds;      // the middle of the tile's first line
+                    k++;
+                } else if (!pack(all, p, centre)) {
+                    break;
+                }
+                compute(g, p, ds, centre);
+            }
+            tile += nk;
+        }
+        return next;
+    }
+
+    // ---- scan ----
+    // Rows: warp w takes the unit's tile w, its positions 32 at a time; match[state][w][i] is the ballot
+    // of positions 32 i .. 32 i + 31 of the tile (positions past its end count as matching).
+    __device__ __forceinline__ void scan_rows(const AxisGeom<T>& g, int tile0, int nk, bool v0, bool v1)
+    {
+        const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        if (w >= nk) return;
+        int seg, grp;
+        place(g, tile0 + w, seg, grp);
+        if (grp >= g.nlines) return;
+        const int a0 = seg * g.tile_len;
+        const int width = min(g.n, a0 + g.tile_len) - a0 + 2 * H;
+        const int64_t base = A.origin + (int64_t)grp * g.lstride;
+        constexpr int kBatch = sizeof(T) == 8 ? 4 : 8;
+#pragma unroll
+        for (int i0 = 0; i0 < kTileWarps; i0 += kBatch) {
+            CellIn<T> c[kBatch];
+#pragma unroll
+            for (int i = 0; i < kBatch; i++) {
+                c[i] = CellIn<T>{};
+                const int q = 32 * (i0 + i) + lane;
+                if (q < width) {
+                    int m, side;
+                    source(g.n, a0 - H + q, m, side);
+                    load(base + m, c[i]);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < kBatch; i++) {
+                const int q = 32 * (i0 + i) + lane;
+                int m, side;
+                const bool stale = source(g.n, a0 - H + q, m, side);
+                mirror(g, c[i], side);
+                const bool out = q >= width;
+                const uint32_t b0 = __ballot_sync(0xffffffffu, out || (v0 && !stale && same_as_kept(c[i], 0)));
+                const uint32_t b1 = __ballot_sync(0xffffffffu, out || (v1 && !stale && same_as_kept(c[i], 1)));
+                if (lane == 0) {
+                    sh.match[parity][0][w][i0 + i] = b0;
+                    sh.match[parity][1][w][i0 + i] = b1;
+                }
+            }
+        }
+        __syncwarp();
+        if (__any_sync(0xffffffffu, chunk_state(w, lane) >= 0 && 8 * lane < width - 2 * H) && lane == 0)
+            sh.uniform[parity] = 1;
+    }
+    // The kept state of chunk j (owned positions 8 j .. 8 j + 7) of warp w's tile, -1 when its windows do
+    // not all hold one: they lie in positions 8 j .. 8 j + 15 of the tile.
+    __device__ __forceinline__ int chunk_state(int w, int j) const
+    {
+        if (j >= 31) return -1;
+        const uint16_t b0 = window16(&sh.match[parity][0][w][0], j), b1 = window16(&sh.match[parity][1][w][0], j);
+        return b0 == 0xffffu ? 0 : b1 == 0xffffu ? 1 : -1;
+    }
+    static __device__ __forceinline__ uint16_t window16(const uint32_t* words, int j)
+    {
+        const unsigned char* b = reinterpret_cast<const unsigned char*>(words);
+        return (uint16_t)(b[j] | (b[j + 1] << 8));
+    }
+    __device__ __forceinline__ void fill_rows(const AxisGeom<T>& g, int tile0, int nk)
+    {
+        const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        if (w >= nk) return;
+        int seg, grp;
+        place(g, tile0 + w, seg, grp);
+        if (grp >= g.nlines) return;
+        const int a0 = seg * g.tile_len;
+        const int len = min(g.n, a0 + g.tile_len) - a0;
+        const int e = chunk_state(w, lane);
+        const uint32_t live = __ballot_sync(0xffffffffu, 8 * lane < len);
+        const uint32_t idle0 = __ballot_sync(0xffffffffu, e == 0), idle1 = __ballot_sync(0xffffffffu, e == 1);
+        push(live & ~(idle0 | idle1), grp, a0, len);
+        const int64_t base = A.origin + (int64_t)grp * g.lstride + a0;
+        for (int o = lane; o < len; o += 32) {
+            const int j = o >> 3;
+            if ((idle0 >> j) & 1u) store_kept(base + o, 0);
+            else if ((idle1 >> j) & 1u) store_kept(base + o, 1);
+        }
+    }
+    // Appends the runs of a line's chunks in `todo` (bit j: chunk j, at a0 + 8 j) to the list; runs one
+    // idle chunk apart are joined (they share their halos).  Every lane of a warp has the same mask.
+    __device__ __forceinline__ void push(uint32_t todo, int line, int a0, int len)
+    {
+        todo |= (todo << 1) & (todo >> 1);
+        const int lane = threadIdx.x & 31;
+        if (((todo >> lane) & 1u) && (lane == 0 || !((todo >> (lane - 1)) & 1u))) push_run(todo >> lane, lane, line, a0, len);
+    }
+    __device__ __forceinline__ void push_run(uint32_t mask, int j, int line, int a0, int len)
+    {
+        const int chunks = __ffs((int)~mask) - 1;            // ones at the low end (mask has at most 31)
+        const int cells = min(8 * chunks, len - 8 * j);
+        const uint32_t at = atomicAdd(&sh.tail[parity], 1u);
+        sh.list[at % kTileList] = Stretch{line, ((a0 + 8 * j) << 8) | cells};
+    }
+    __device__ __forceinline__ void store_kept(int64_t i, int e)
+    {
+        const T* kv = sh.kept[e];
+        T* const* out = A.buf[src ^ 1];
+        out[0][i] = kv[kRunOut];
+        out[1 + axis][i] = kv[kRunOut + 1];
+        out[2 - axis][i] = kv[kRunOut + 2];
+        out[3][i] = kv[kRunOut + 3];
+        if (pcg) {
+            A.pmat[i] = kv[kRunP];
+            A.cmat[i] = kv[kRunC];
+            A.gmat[i] = (1 + A.gamma) / 2;
+        }
+    }
+    // Columns: the unit's tiles are columns line0 .. of one segment, a lane each; warp w takes positions
+    // 8 w .. 8 w + 7 of the segment (halo included), and match[state][0][w] has bit c set when they all
+    // match in column c.  Chunk j of a column is uniform when words j and j + 1 have its bit.
+    __device__ __forceinline__ void scan_columns(const AxisGeom<T>& g, int tile0, int nk, bool v0, bool v1)
+    {
+        const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        int seg, grp;
+        place(g, tile0, seg, grp);
+        const int line = grp * g.tile_lines + lane;
+        const bool col = lane < nk * g.tile_lines && line < g.nlines;
+        const int a0 = seg * g.tile_len;
+        const int width = min(g.n, a0 + g.tile_len) - a0 + 2 * H;
+        const int64_t base = A.origin + (int64_t)line * g.lstride;
+        constexpr int kBatch = sizeof(T) == 8 ? 4 : 8;
+        bool m0 = v0, m1 = v1;
+        if (col) {
+#pragma unroll
+            for (int i0 = 0; i0 < 8; i0 += kBatch) {
+                CellIn<T> c[kBatch];
+#pragma unroll
+                for (int i = 0; i < kBatch; i++) {
+                    c[i] = CellIn<T>{};
+                    const int q = 8 * w + i0 + i;
+                    if (q < width) {
+                        int m, side;
+                        source(g.n, a0 - H + q, m, side);
+                        load(base + (int64_t)m * g.s, c[i]);
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < kBatch; i++) {
+                    const int q = 8 * w + i0 + i;
+                    if (q < width) {
+                        int m, side;
+                        const bool stale = source(g.n, a0 - H + q, m, side);
+                        mirror(g, c[i], side);
+                        m0 = m0 && !stale && same_as_kept(c[i], 0);
+                        m1 = m1 && !stale && same_as_kept(c[i], 1);
+                    }
+                }
+            }
+        }
+        const uint32_t b0 = __ballot_sync(0xffffffffu, m0), b1 = __ballot_sync(0xffffffffu, m1);
+        if (lane == 0) {
+            sh.match[parity][0][0][w] = b0;
+            sh.match[parity][1][0][w] = b1;
+        }
+        __syncthreads();
+        if (w < kTileWarps - 1) {
+            const uint32_t idle = (sh.match[parity][0][0][w] & sh.match[parity][0][0][w + 1]) |
+                                  (sh.match[parity][1][0][w] & sh.match[parity][1][0][w + 1]);
+            if (__any_sync(0xffffffffu, col && ((idle >> lane) & 1u) && 8 * w < width - 2 * H) && lane == 0)
+                sh.uniform[parity] = 1;
+        }
+    }
+    __device__ __forceinline__ void fill_columns(const AxisGeom<T>& g, int tile0, int nk)
+    {
+        const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        int seg, grp;
+        place(g, tile0, seg, grp);
+        const int line = grp * g.tile_lines + lane;
+        const bool col = lane < nk * g.tile_lines && line < g.nlines;
+        const int a0 = seg * g.tile_len;
+        const int len = min(g.n, a0 + g.tile_len) - a0;
+        const uint32_t* M0 = &sh.match[parity][0][0][0];
+        const uint32_t* M1 = &sh.match[parity][1][0][0];
+        if (w < kTileWarps - 1) {
+            // warp w stores chunk w of the uniform columns
+            const int e = !col ? -1 : ((M0[w] & M0[w + 1]) >> lane) & 1u ? 0 : ((M1[w] & M1[w + 1]) >> lane) & 1u ? 1 : -1;
+            if (e >= 0) {
+                const int end = min(8 * w + 8, len);
+                for (int o = 8 * w; o < end; o++) store_kept(A.origin + (int64_t)line * g.lstride + (int64_t)(a0 + o) * g.s, e);
+            }
+        } else if (col) {
+            // the last warp lists the others' chunks, a lane per column
+            uint32_t todo = 0;
+            for (int j = 0; 8 * j < len; j++)
+                if (!((((M0[j] & M0[j + 1]) | (M1[j] & M1[j + 1])) >> lane) & 1u)) todo |= 1u << j;
+            todo |= (todo << 1) & (todo >> 1);
+            for (int j = 0; todo >> j; j++)
+                if (((todo >> j) & 1u) && (j == 0 || !((todo >> (j - 1)) & 1u))) push_run(todo >> j, j, line, a0, len);
+        }
+    }
+
+    // ---- packed stretches ----
+    // The thread's place among the list's next stretches, as many as fit in the block; false when the
+    // list is empty or (unless `all`) would leave a quarter of the threads idle.
+    __device__ __forceinline__ bool pack(bool all, Spot& p, int& centre)
+    {
+        const int tid = threadIdx.x, lane = tid & 31;
+        const uint32_t head = sh.head;
+        const int left = (int)(sh.tail[parity] - head);
+        if (left == 0) return false;
+        // every warp packs for itself: inclusive sums of the next 32 stretches' threads
+        Stretch s{0, 0};
+        int need = 1 << 20;
+        if (lane < left) {
+            s = sh.list[(head + lane) % kTileList];
+            need = (s.start_len & 255) + 2 * H;
+        }
+        int sum = need;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, sum, o);
+            if (lane >= o) sum += v;
+        }
+        const int take = __popc(__ballot_sync(0xffffffffu, sum <= kTileThreads));
+        if (!all && take == left && __shfl_sync(0xffffffffu, sum, take - 1) < kTileThreads * 3 / 4) return false;
+        // this thread's stretch: the first whose sum lies above its index
+        int k = 0;
+        for (int o = 16; o > 0; o >>= 1) {
+            const int v = __shfl_sync(0xffffffffu, sum, k + o - 1);
+            if (v <= tid) k += o;
+        }
+        const int line = __shfl_sync(0xffffffffu, s.line, k);
+        const int sl = __shfl_sync(0xffffffffu, s.start_len, k);
+        p.q = tid - __shfl_sync(0xffffffffu, sum - need, k);
+        p.width = (sl & 255) + 2 * H;
+        p.t = (sl >> 8) - H + p.q;
+        p.base = A.origin + (int64_t)line * A.geom[axis].lstride;
+        p.in = k < take;
+        centre = (__shfl_sync(0xffffffffu, s.start_len, 0) & 255) / 2 + H;
+        __syncthreads();         // before sh.head or the entries are written again
+        if (tid == 0) sh.head = head + take;
+        return true;
+    }
+
+    // ---- compute ----
+    // The kept-state slot that the centre thread's state may take, -1 when it should not be recorded:
+    // its window is not real and uniform, or the state is kept already.  Run by the centre's warp.
+    __device__ __forceinline__ int claim_slot(const AxisGeom<T>& g, const Spot& p, const CellIn<T>& c, int centre)
+    {
+        const int lane = threadIdx.x & 31, from = centre & 31;
+        const int tc = __shfl_sync(0xffffffffu, p.t, from);
+        const int in = __shfl_sync(0xffffffffu, (int)p.in, from);
+        if (!in || tc - H < 0 || tc + H >= g.n) return -1;
+        const int64_t bc = __shfl_sync(0xffffffffu, (long long)p.base, from);
+        CellIn<T> u;
+        u.rho = __shfl_sync(0xffffffffu, c.rho, from);
+        u.ua = __shfl_sync(0xffffffffu, c.ua, from);
+        u.uo = __shfl_sync(0xffffffffu, c.uo, from);
+        u.E = __shfl_sync(0xffffffffu, c.E, from);
+        bool same = true;
+        if (lane <= 2 * H) {
+            CellIn<T> o;
+            load(bc + (int64_t)(tc - H + lane) * g.s, o);
+            same = same_state(o, u);
+        }
+        if (!__all_sync(0xffffffffu, same)) return -1;
+        const bool v0 = sh.valid[0] != 0, v1 = sh.valid[1] != 0;
+        if ((v0 && same_as_kept(u, 0)) || (v1 && same_as_kept(u, 1))) return -1;
+        const int s = !v0 ? 0 : !v1 ? 1 : sh.turn;
+        __syncwarp();
+        if (lane == 0) {
+            sh.valid[s] = 0;
+            sh.turn = s ^ 1;
+        }
+        __syncwarp();
+        return s;
+    }
+
+    // The stages at the thread's position; ds threads between neighbouring positions.  The centre
+    // thread records its state when it can.
+    __device__ __forceinline__ void compute(const AxisGeom<T>& g, const Spot& p, const int ds, const int centre)
+    {
+        const int tid = threadIdx.x;
+        const T dx = g.dx;
+        const int q = p.q, width = p.width;
+        const bool on = p.in;
+        const bool own = on && q >= H && q < width - H;
+        T* X = &sh.ex[0][tid];
+#define ARMON_X(slot) X[(slot) * kTileThreads]
+#define ARMON_AT(slot, off) X[(slot) * kTileThreads + (off)]
+        int rec = -1;
+
+        // ---- cell: load, mirror, EOS ----
+        CellIn<T> c{};
+        if (on) {
+            int m, side;
+            const bool stale = source(g.n, p.t, m, side);
+            const int64_t i = p.base + (int64_t)m * g.s;
+            load(i, c);
+            mirror(g, c, side);
+            if (stale) {
+                c.p = A.pmat[i];
+                c.c = A.cmat[i];
+            } else {
+                eos(c, A.gamma, A.gamma - 1);
+                if (pcg && own) {
+                    A.pmat[i] = c.p;
+                    A.cmat[i] = c.c;
+                    A.gmat[i] = (1 + A.gamma) / 2;
+                }
+            }
+            c.rc = qmul<1>(c.rho, c.c);
+            c.rcu = qmul<1>(c.rc, c.ua);
+            c.dm = mul_dx(c.rho, g);
+            ARMON_X(9) = c.rc;
+            ARMON_X(10) = c.rcu;
+            ARMON_X(11) = c.p;
+            ARMON_X(12) = c.ua;
+            ARMON_X(13) = c.dm;
+            sh.c[tid] = c.c;
+        }
+        if (A.reuse && g.tile_scan && (tid >> 5) == (centre >> 5)) {
+            rec = claim_slot(g, p, c, centre);
+            if (tid != centre) rec = -1;
+            if (rec >= 0) {
+                T* const rv = sh.kept[rec];
+                rv[kRunRho] = c.rho; rv[kRunUa] = c.ua; rv[kRunUo] = c.uo; rv[kRunE] = c.E;
+                rv[kRunP] = c.p; rv[kRunC] = c.c;
+            }
+        }
+        __syncthreads();
+
+        // ---- Godunov face q (between positions q - 1 and q) ----
+        God<T> G{};
+        GadDiff<T> D{};
+        if (on && q >= 1) {
+            CellIn<T> cl{};
+            cl.rc = ARMON_AT(9, -ds);
+            cl.rcu = ARMON_AT(10, -ds);
+            cl.p = ARMON_AT(11, -ds);
+            cl.ua = ARMON_AT(12, -ds);
+            G = godunov(cl, c);
+            if (kGAD) {
+                D = gad_diff(G, cl, c);
+                ARMON_X(5) = D.au;
+                ARMON_X(6) = D.bu;
+                ARMON_X(7) = D.ap;
+                ARMON_X(8) = D.bp;
+            }
+        }
+        if (kGAD) __syncthreads();
+
+        // ---- flux at face q ----
+        Flux<T> F{};
+        if (on && (kGAD ? (q >= 2 && q <= width - 2) : q >= 1)) {
+            if (kGAD) {
+                GadDiff<T> Dm{}, Dp{};
+                Dm.bu = ARMON_AT(6, -ds);
+                Dm.bp = ARMON_AT(8, -ds);
+                Dp.au = ARMON_AT(5, ds);
+                Dp.ap = ARMON_AT(7, ds);
+                F = gad(G, Dm, D, Dp, ARMON_AT(13, -ds), c.dm, A.limiter, dt);
+            } else {
+                F.us = G.us;
+                F.ps = G.ps;
+            }
+            F.psus = qmul<4>(F.ps, F.us);
+            F.dtus = qmul<4>(dt, F.us);
+            ARMON_X(0) = F.us;
+            ARMON_X(1) = F.ps;
+            ARMON_X(2) = F.psus;
+            ARMON_X(3) = F.dtus;
+        }
+        __syncthreads();
+
+        // ---- Lagrangian cell q (faces q and q + 1) ----
+        Lag<T> L{};
+        const bool has_lag = on && q >= kLagLo && q <= width - 1 - kLagLo;
+        if (has_lag) {
+            Flux<T> F1{};
+            F1.us = ARMON_AT(0, ds);
+            F1.ps = ARMON_AT(1, ds);
+            F1.psus = ARMON_AT(2, ds);
+            L = lagrange(c, F, F1, dt, dx);
+            ARMON_X(4) = L.rho;
+            ARMON_X(5) = L.rua;
+            ARMON_X(6) = L.ruo;
+            ARMON_X(7) = L.rE;
+            ARMON_X(8) = L.W;
+        }
+        __syncthreads();
+
+        // ---- differences of adjacent Lagrangian cells, which two faces share ----
+        if (kE2) {
+            if (has_lag && q >= kLagLo + 1) {
+                Lag<T> Lm{};
+                Lm.rho = ARMON_AT(4, -ds);
+                Lm.rua = ARMON_AT(5, -ds);
+                Lm.ruo = ARMON_AT(6, -ds);
+                Lm.rE = ARMON_AT(7, -ds);
+                const Adv<T> d = lag_diff(Lm, L);
+                ARMON_X(9) = d.r;
+                ARMON_X(10) = d.ra;
+                ARMON_X(11) = d.ro;
+                ARMON_X(12) = d.rE;
+                ARMON_X(13) = ARMON_AT(8, -ds) + L.W;
+            }
+            __syncthreads();
+        }
+
+        // ---- advection flux at face q ----
+        Adv<T> a{};
+        if (on && q >= H && q <= width - H) {
+            const T disp = F.dtus;
+            const bool up = qgt0(disp);
+            const int o = up ? -ds : 0;       // the upwind cell
+            if (kE2) {
+                const T Dx = qneg_if(dx + (up ? qneg_if(ARMON_AT(3, -ds), true) : ARMON_AT(3, ds)), up);
+                const Adv<T> u0{ARMON_AT(4, o), ARMON_AT(5, o), ARMON_AT(6, o), ARMON_AT(7, o)};
+                const Adv<T> dm{ARMON_AT(9, o), ARMON_AT(10, o), ARMON_AT(11, o), ARMON_AT(12, o)};
+                const int o1 = o + ds;
+                const Adv<T> dp{ARMON_AT(9, o1), ARMON_AT(10, o1), ARMON_AT(11, o1), ARMON_AT(12, o1)};
+                a = advect2_upwind(disp, Dx, ARMON_AT(8, o), u0, dm, dp, ARMON_AT(13, o), ARMON_AT(13, o1));
+            } else {
+                a.r = qmul<6>(disp, ARMON_AT(4, o));
+                a.ra = qmul<6>(disp, ARMON_AT(5, o));
+                a.ro = qmul<6>(disp, ARMON_AT(6, o));
+                a.rE = qmul<6>(disp, ARMON_AT(7, o));
+            }
+            ARMON_X(0) = a.r;
+            ARMON_X(1) = a.ra;
+            ARMON_X(2) = a.ro;
+            ARMON_X(14) = a.rE;
+        }
+        if (rec >= 0) sh.valid[rec] = 1;    // its results follow; they are read after the next unit's first barrier
+        __syncthreads();
+
+        // ---- projection of cell q (src/kernels/euler_projection.cpp:36-46) ----
+        if (own) {
+            const T dXr = qmul<7>(L.W, L.rho);
+            T o[4];
+            o[0] = div_dx(dXr - (ARMON_AT(0, ds) - a.r), g);
+            const T ra = div_dx(qmul<7>(dXr, L.ua) - (ARMON_AT(1, ds) - a.ra), g);
+            const T ro = div_dx(qmul<7>(dXr, L.uo) - (ARMON_AT(2, ds) - a.ro), g);
+            const T rE = div_dx(qmul<7>(dXr, L.E) - (ARMON_AT(14, ds) - a.rE), g);
+            const auto inv_rho = qrecip_at<8>(o[0]);
+            o[1] = qdiv_at<8>(ra, inv_rho);
+            o[2] = qdiv_at<8>(ro, inv_rho);
+            o[3] = qdiv_at<8>(rE, inv_rho);
+            const int64_t i = p.base + (int64_t)p.t * g.s;
+            T* const* out = A.buf[src ^ 1];
+            out[0][i] = o[0];
+            out[1 + axis][i] = o[1];
+            out[2 - axis][i] = o[2];
+            out[3][i] = o[3];
+            if (last) {
+                // dt_CFL of the state after this pass, with c from this pass's EOS; a kept state was
+                // recorded by a thread that adds it here
+                if (axis == 0) sh.acc[tid].add(o[1], o[2], sh.c[tid]);
+                else sh.acc[tid].add(o[2], o[1], sh.c[tid]);
+            }
+            if (rec >= 0) {
+                T* const rv = sh.kept[rec];
+                rv[kRunOut] = o[0]; rv[kRunOut + 1] = o[1]; rv[kRunOut + 2] = o[2]; rv[kRunOut + 3] = o[3];
+            }
+        }
+#undef ARMON_X
+#undef ARMON_AT
+    }
+};
+
+// Adds the block's dt maxima to the domain's (max_x, max_y of its state).  Every thread calls it.
+template <class T>
+__device__ __forceinline__ void tile_flush(TileShared<T>& sh, StepState* state)
+{
+    __shared__ unsigned long long red[2];
+    const int tid = threadIdx.x;
+    if (tid < 2) red[tid] = 0;
+    __syncthreads();
+    DtAcc acc = sh.acc[tid];
+    acc.finish();
+    for (int o = 16; o > 0; o >>= 1)
+        acc.merge(__shfl_xor_sync(0xffffffffu, acc.ax, o), __shfl_xor_sync(0xffffffffu, acc.ay, o));
+    if ((tid & 31) == 0) {
+        // maxima of non-negative, non-NaN values: the order of the bit patterns
+        atomicMax(&red[0], (unsigned long long)__double_as_longlong(acc.ax));
+        atomicMax(&red[1], (unsigned long long)__double_as_longlong(acc.ay));
+    }
+    __syncthreads();
+    if (tid == 0) {
+        if (red[0] > __ldcg((const unsigned long long*)&state->max_x)) atomicMax((unsigned long long*)&state->max_x, red[0]);
+        if (red[1] > __ldcg((const unsigned long long*)&state->max_y)) atomicMax((unsigned long long*)&state->max_y, red[1]);
+    }
+    sh.acc[tid].init();
+}
+
+// The end of a cycle for one domain: dt_CFL, time and cycle (run by one thread when every block of the
+// launch has added its maxima).
+static __device__ __forceinline__ void tile_commit(StepState* state, const StepConfig& cfg)
+{
+    StepState st;
+    st.time = __ldcg(&state->time);
+    st.current_dt = __ldcg(&state->current_dt);
+    st.next_dt = __ldcg(&state->next_dt);
+    st.raw_dt = __ldcg(&state->raw_dt);
+    st.cycle = __ldcg(&state->cycle);
+    st.status = __ldcg(&state->status);
+    st.counter = 0;
+    st.buf_base = __ldcg(&state->buf_base);
+    const double ax = __longlong_as_double((long long)__ldcg((const unsigned long long*)&state->max_x));
+    const double ay = __longlong_as_double((long long)__ldcg((const unsigned long long*)&state->max_y));
+    const CycleDt cd = cycle_time_step(st, cfg);
+    if (!cd.run || cd.invalid) return;
+    st.raw_dt = dt_from_maxima(ax, ay, cfg.dt_dx, cfg.dt_dy);
+    st.current_dt = cd.current;
+    st.next_dt = cd.next;
+    st.time += cd.current;
+    st.cycle += 1;
+    st.max_x = st.max_y = 0;
+    *state = st;
+}
+
+// Whether this block is the launch's last to get here; resets the launch's counters then.
+__device__ __forceinline__ bool tile_arrive(TileCtl* ctl)
+{
+    __shared__ int is_last;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        is_last = atomicAdd(&ctl->arrived, 1u) == gridDim.x - 1;
+        if (is_last) {
+            ctl->ticket = 0;
+            ctl->arrived = 0;
+            __threadfence();
+        }
+    }
+    __syncthreads();
+    return is_last != 0;
+}
+
+template <class T>
+__device__ __forceinline__ void tile_forget(TileShared<T>& sh)
+{
+    if (threadIdx.x == 0) {
+        sh.valid[0] = sh.valid[1] = 0;
+        sh.turn = 0;
+        sh.head = sh.tail[0] = sh.tail[1] = 0;
+        sh.uniform[0] = sh.uniform[1] = 0;
+    }
+}
+
+// One domain.
+template <class T, int SCHEME, int PROJ>
+__global__ void __launch_bounds__(kTileThreads, tile_min_blocks<T>())
+tile_kernel(const __grid_constant__ SweepArgs<T> A, TileCtl* ctl, int last)
+{
+    __shared__ TileShared<T> sh;
+    TilePass<T, SCHEME, PROJ> P(A, sh);
+    tile_forget(sh);
+    sh.acc[threadIdx.x].init();
+    if (P.start(A.pass, last != 0, blockIdx.x == 0 && threadIdx.x == 0)) {
+        const int total = A.geom[P.axis].tile_units;
+        __syncthreads();
+        int u = blockIdx.x;
+        while (u < total) {
+            u = P.unit(u, total, [&]() {
+                return total > (int)gridDim.x ? (int)(gridDim.x + atomicAdd(&ctl->ticket, 1u)) : total;
+            });
+        }
+        if (last) tile_flush(sh, A.state);
+    }
+    if (tile_arrive(ctl) && last && threadIdx.x == 0) tile_commit(A.state, A.cfg);
+}
+
+}  // namespace armon
