@@ -148,6 +148,10 @@ __host__ __device__ __forceinline__ uint64_t quot_estimate(uint64_t ma, uint64_t
     return ((uint64_t)q1 << 26) + q2;
 }
 
+// The FP64 division of the operands that the integer path leaves, out of line: inlined at every
+// division it would be a fifth of a pass's code.
+static __device__ __noinline__ double div_hw(double a, double b) { return a / b; }
+
 // a / b; the reciprocal comes from get_y(mb), called only on the integer path.
 template <class GetY>
 __device__ __forceinline__ double div_core(double a, double b, uint64_t ub, GetY get_y)
@@ -160,7 +164,7 @@ __device__ __forceinline__ double div_core(double a, double b, uint64_t ub, GetY
     const bool b_normal = (eb - 1u) < 2046u;
     if (!(b_normal && (ea - 1u) < 2046u && (unsigned)(e0 + 1021) <= 2043u)) {
         if (b_normal && (ua << 1) == 0) return from_bits(sign);   // +-0 / normal
-        return a / b;
+        return div_hw(a, b);
     }
     uint64_t ma = (ua & kMant) | kHidden;
     const uint64_t mb = (ub & kMant) | kHidden;
@@ -175,7 +179,10 @@ __device__ __forceinline__ double div_core(double a, double b, uint64_t ub, GetY
     return from_bits(sign + ((uint64_t)(uint32_t)(e0 + 1022 - (int)less) << 52) + q);
 }
 
-__device__ __forceinline__ double div(double a, double b)
+#ifndef DIVATTR
+#define DIVATTR __forceinline__
+#endif
+static __device__ DIVATTR double div(double a, double b)
 {
     return div_core(a, b, bits(b), [](uint64_t mb) { return recip_y(mb); });
 }
@@ -316,11 +323,13 @@ __device__ __forceinline__ double add(double a, double b)
 // 2^64, exact because |R| < 2^58 for an estimate within a few units); if R is still outside
 // [0, 2Q] the hardware square root is used.  Zeros are returned as they are; negative, subnormal,
 // infinite and NaN operands take the hardware square root.
+static __device__ __noinline__ double sqrt_hw(double x) { return ::sqrt(x); }
+
 __device__ __forceinline__ double sqrt(double x)
 {
     const uint64_t u = bits(x);
     const uint32_t e = (uint32_t)(u >> 52);                  // sign and exponent
-    if (e - 1u >= 2046u) return (u << 1) == 0 ? x : ::sqrt(x);
+    if (e - 1u >= 2046u) return (u << 1) == 0 ? x : sqrt_hw(x);
     const uint32_t odd = (e & 1u) ^ 1u;                      // e - 1075 is odd
     const uint64_t M = ((u & kMant) | kHidden) << odd;       // [2^52, 2^54)
     const uint64_t A = M << 10;                              // a in Q62
@@ -352,7 +361,7 @@ __device__ __forceinline__ double sqrt(double x)
         R -= up ? (int64_t)(2 * Q + 1) : 0;
         Q += up ? 1u : 0u;
     }
-    if (R < 0 || R > (int64_t)(2 * Q)) return ::sqrt(x);   // outside the error bounds
+    if (R < 0 || R > (int64_t)(2 * Q)) return sqrt_hw(x);   // outside the error bounds
     Q += R > (int64_t)Q ? 1u : 0u;
     const int be = ((int)e - 1075 - (int)odd) / 2 + 1049;          // biased exponent of the result
     return from_bits(((uint64_t)(be - 1) << 52) + Q);

@@ -339,7 +339,7 @@ __device__ __forceinline__ double limited_ratio(int L, double num, double den)
         if (an < sfp::kInf && ad < sfp::kInf && ad != 0) {
             if (an == 0 || ((un ^ ud) >> 63)) return 0.0;
             if (an >= ad) return 1.0;
-            return qdiv_at<2>(num, den);     // in (0, 1]: min(1, .) and max(0, .) keep it
+            // else a quotient in (0, 1], which min(1, .) and max(0, .) keep
         }
     }
     return limiter_fn(L, qdiv_at<2>(num, den));

@@ -258,6 +258,8 @@ struct TilePass {
     }
 
     // ---- scan ----
+    // Ghosts never match (their mirrored velocities differ from a state at rest by the sign of zero), so
+    // the chunks next to a wall are computed.
     // Rows: warp w takes the unit's tile w, its positions 32 at a time; match[state][w][i] is the ballot
     // of positions 32 i .. 32 i + 31 of the tile (positions past its end count as matching).
     __device__ __forceinline__ void scan_rows(const AxisGeom<T>& g, int tile0, int nk, bool v0, bool v1)
@@ -271,28 +273,21 @@ struct TilePass {
         const int width = min(g.n, a0 + g.tile_len) - a0 + 2 * H;
         const int64_t base = A.origin + (int64_t)grp * g.lstride;
         constexpr int kBatch = sizeof(T) == 8 ? 4 : 8;
-#pragma unroll
+#pragma unroll 1
         for (int i0 = 0; i0 < kTileWarps; i0 += kBatch) {
             CellIn<T> c[kBatch];
 #pragma unroll
             for (int i = 0; i < kBatch; i++) {
                 c[i] = CellIn<T>{};
-                const int q = 32 * (i0 + i) + lane;
-                if (q < width) {
-                    int m, side;
-                    source(g.n, a0 - H + q, m, side);
-                    load(base + m, c[i]);
-                }
+                const int q = 32 * (i0 + i) + lane, t = a0 - H + q;
+                if (q < width && t >= 0 && t < g.n) load(base + t, c[i]);
             }
 #pragma unroll
             for (int i = 0; i < kBatch; i++) {
-                const int q = 32 * (i0 + i) + lane;
-                int m, side;
-                const bool stale = source(g.n, a0 - H + q, m, side);
-                mirror(g, c[i], side);
-                const bool out = q >= width;
-                const uint32_t b0 = __ballot_sync(0xffffffffu, out || (v0 && !stale && same_as_kept(c[i], 0)));
-                const uint32_t b1 = __ballot_sync(0xffffffffu, out || (v1 && !stale && same_as_kept(c[i], 1)));
+                const int q = 32 * (i0 + i) + lane, t = a0 - H + q;
+                const bool out = q >= width, real = t >= 0 && t < g.n;
+                const uint32_t b0 = __ballot_sync(0xffffffffu, out || (v0 && real && same_as_kept(c[i], 0)));
+                const uint32_t b1 = __ballot_sync(0xffffffffu, out || (v1 && real && same_as_kept(c[i], 1)));
                 if (lane == 0) {
                     sh.match[parity][0][w][i0 + i] = b0;
                     sh.match[parity][1][w][i0 + i] = b1;
@@ -381,29 +376,21 @@ struct TilePass {
         constexpr int kBatch = sizeof(T) == 8 ? 4 : 8;
         bool m0 = v0, m1 = v1;
         if (col) {
-#pragma unroll
+#pragma unroll 1
             for (int i0 = 0; i0 < 8; i0 += kBatch) {
                 CellIn<T> c[kBatch];
 #pragma unroll
                 for (int i = 0; i < kBatch; i++) {
                     c[i] = CellIn<T>{};
-                    const int q = 8 * w + i0 + i;
-                    if (q < width) {
-                        int m, side;
-                        source(g.n, a0 - H + q, m, side);
-                        load(base + (int64_t)m * g.s, c[i]);
-                    }
+                    const int q = 8 * w + i0 + i, t = a0 - H + q;
+                    if (q < width && t >= 0 && t < g.n) load(base + (int64_t)t * g.s, c[i]);
                 }
 #pragma unroll
                 for (int i = 0; i < kBatch; i++) {
-                    const int q = 8 * w + i0 + i;
-                    if (q < width) {
-                        int m, side;
-                        const bool stale = source(g.n, a0 - H + q, m, side);
-                        mirror(g, c[i], side);
-                        m0 = m0 && !stale && same_as_kept(c[i], 0);
-                        m1 = m1 && !stale && same_as_kept(c[i], 1);
-                    }
+                    const int q = 8 * w + i0 + i, t = a0 - H + q;
+                    const bool out = q >= width, real = t >= 0 && t < g.n;
+                    m0 = m0 && (out || (real && same_as_kept(c[i], 0)));
+                    m1 = m1 && (out || (real && same_as_kept(c[i], 1)));
                 }
             }
         }
