@@ -179,10 +179,16 @@ __device__ __forceinline__ double div_core(double a, double b, uint64_t ub, GetY
     return from_bits(sign + ((uint64_t)(uint32_t)(e0 + 1022 - (int)less) << 52) + q);
 }
 
-#ifndef DIVATTR
-#define DIVATTR __forceinline__
+// Out of line in the translation units that define ARMON_SFP_CALLS: the tile pass (sweep_tile.cuh), whose
+// warps run every stage on few positions each, waits on instruction fetch when its code is larger
+// (4096x4096 circular Sod, 200 cycles: 210 ms inline, 201 ms out of line; a 2048x2048 moving flow 47.9
+// and 47.4 ms).  The marches keep it inline.
+#ifdef ARMON_SFP_CALLS
+#define ARMON_SFP_DIV __noinline__
+#else
+#define ARMON_SFP_DIV __forceinline__
 #endif
-static __device__ DIVATTR double div(double a, double b)
+static __device__ ARMON_SFP_DIV double div(double a, double b)
 {
     return div_core(a, b, bits(b), [](uint64_t mb) { return recip_y(mb); });
 }
@@ -213,28 +219,42 @@ __device__ __forceinline__ double div(double a, const Recip& R, double b)
 // everything below (a sticky bit); round to nearest, ties to even.  Zero operands give signed zeros;
 // subnormal, infinite and NaN operands and results near or outside the ends of the normal range
 // take the FP64 multiply.
-__device__ __forceinline__ double mul(double a, double b)
+// the other operands, out of line
+static __device__ __noinline__ double mul_rest(double a, double b)
 {
     const uint64_t ua = bits(a), ub = bits(b);
-    const uint32_t ea = (uint32_t)(ua >> 52) & 0x7FFu;
-    const uint32_t eb = (uint32_t)(ub >> 52) & 0x7FFu;
+    const uint32_t ea = (uint32_t)(ua >> 52) & 0x7FFu, eb = (uint32_t)(ub >> 52) & 0x7FFu;
     const uint64_t sign = (ua ^ ub) & ~kAbs;
-    const uint32_t e = ea + eb - 1024u;      // the result's biased exponent less one, before normalisation
-    if ((ea - 1u) < 2046u && (eb - 1u) < 2046u && e < 2044u) {
-        const uint64_t xa = ((ua & kMant) | kHidden) << 11;
-        const uint64_t xb = ((ub & kMant) | kHidden) << 11;
-        const unsigned __int128 p = (unsigned __int128)xa * xb;
-        const uint64_t hi = (uint64_t)(p >> 64), lo = (uint64_t)p;
-        const uint32_t top = (uint32_t)(hi >> 63);
-        const uint64_t w = (top ? hi : (hi << 1) | (lo >> 63)) | (lo != 0 ? 1u : 0u);
-        const uint64_t m = w >> 11;
-        const uint32_t up = ((uint32_t)w & 0x7FFu) + ((uint32_t)m & 1u) > 0x400u ? 1u : 0u;
-        return from_bits(sign + ((uint64_t)(e + top) << 52) + m + up);
-    }
     if (((ua << 1) == 0 && (eb - 1u) < 2046u) || ((ub << 1) == 0 && (ea - 1u) < 2046u) ||
         ((ua << 1) == 0 && (ub << 1) == 0))
         return from_bits(sign);                                  // +-0 * normal or zero
     return a * b;
+}
+__device__ __forceinline__ double mul(double a, double b)
+{
+    const uint64_t ua = bits(a), ub = bits(b);
+    const uint32_t ah = (uint32_t)(ua >> 32), bh = (uint32_t)(ub >> 32), al = (uint32_t)ua, bl = (uint32_t)ub;
+    const uint32_t ea = (ah >> 20) & 0x7FFu, eb = (bh >> 20) & 0x7FFu;
+    const uint32_t sign = (ah ^ bh) & 0x80000000u;
+    const uint32_t e = ea + eb - 1024u;      // the result's biased exponent less one, before normalisation
+    if ((ea - 1u) < 2046u && (eb - 1u) < 2046u && e < 2044u) {
+        const uint32_t xh = (ah << 11 | al >> 21) | 0x80000000u, xl = al << 11;
+        const uint32_t yh = (bh << 11 | bl >> 21) | 0x80000000u, yl = bl << 11;
+        const uint64_t p0 = (uint64_t)xl * yl;
+        const uint64_t p1 = (uint64_t)xl * yh + (p0 >> 32);
+        const uint64_t p2 = (uint64_t)xh * yl + (uint32_t)p1;
+        const uint64_t p3 = (uint64_t)xh * yh + (p1 >> 32) + (p2 >> 32);
+        const uint32_t top = (uint32_t)(p3 >> 63);
+        uint32_t wh = (uint32_t)(p3 >> 32), wl = (uint32_t)p3;
+        const uint32_t low = (uint32_t)p2;
+        wh = __funnelshift_l(wl, wh, 1u - top);
+        wl = __funnelshift_l(low, wl, 1u - top) | ((low | (uint32_t)p0) != 0 ? 1u : 0u);
+        const uint32_t ml = __funnelshift_r(wl, wh, 11);
+        const uint32_t up = (wl & 0x7FFu) + (ml & 1u) > 0x400u ? 1u : 0u;
+        const uint64_t m = ((uint64_t)(sign + ((e + top) << 20) + (wh >> 11)) << 32 | ml) + up;
+        return from_bits(m);
+    }
+    return mul_rest(a, b);
 }
 
 // Addition (my own construction).  For normal operands, x the one of larger magnitude and y the

@@ -37,7 +37,7 @@ struct armon_solver {
     size_t elem = 8;
     void* arr[16] = {};
     bool owns_arrays = false;
-    StepState* d_state = nullptr;   // followed by the tile launches' counters
+    StepState* d_state = nullptr;   // followed by the tile launches' counters and hints
     TileCtl* d_ctl = nullptr;
     StepState* h_state = nullptr;   // pinned
     double* d_partials = nullptr;
@@ -100,6 +100,8 @@ int cuda_fail(cudaError_t e, const char* what)
     } while (0)
 
 constexpr int kTileYLines = 4;
+// the step state, then the tile launches' counters and hints
+constexpr size_t kStateBytes = sizeof(StepState) + sizeof(TileCtl) + sizeof(TileHints<double>);
 
 template <class T>
 void fill_geom(armon_solver* s, SweepArgs<T>& a)
@@ -119,6 +121,7 @@ void fill_geom(armon_solver* s, SweepArgs<T>& a)
         a.face_stride = s->face_stride;
     }
     if (s->tile) {
+        a.hints = reinterpret_cast<TileHints<T>*>(s->d_ctl + 1);
         if (s->tile_per_sm == 0) s->tile_per_sm = sweep_tile_blocks_per_sm(s->fp32, s->p.scheme, s->p.projection);
         const int slots = s->sm_count * s->tile_per_sm;
         int units = 1;
@@ -639,7 +642,7 @@ static int solver_create(const armon_params* p, const armon_solver_opts* opts, d
             }
         }
     }
-    e = cudaMalloc(&s->d_state, sizeof(StepState) + sizeof(TileCtl));
+    e = cudaMalloc(&s->d_state, kStateBytes);
     s->d_ctl = reinterpret_cast<TileCtl*>(s->d_state + 1);
     if (e == cudaSuccess) e = cudaMallocHost(&s->h_state, sizeof(StepState));
     // the partial buffers are sized after the geometry is known
@@ -663,7 +666,7 @@ static int solver_create(const armon_params* p, const armon_solver_opts* opts, d
         }
     }
     s->default_split = s->split;
-    if (e == cudaSuccess) e = cudaMemsetAsync(s->d_state, 0, sizeof(StepState) + sizeof(TileCtl), s->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(s->d_state, 0, kStateBytes, s->stream);
     if (e != cudaSuccess) { armon_solver_destroy(s); return cuda_fail(e, "solver allocation"); }
     std::memset(s->h_state, 0, sizeof(StepState));
     if (s->fp32) fill_geom(s, s->a32); else fill_geom(s, s->a64);
@@ -728,7 +731,7 @@ int armon_solver_begin_loop(armon_solver* s)
     b.cfg = s->cfg;
     b.partials = s->d_partials;
     b.buf_base = 0;
-    CUDA_TRY(cudaMemsetAsync(&s->d_state->counter, 0, sizeof(uint32_t), s->stream));
+    CUDA_TRY(cudaMemsetAsync(s->d_state, 0, kStateBytes, s->stream));
     CUDA_TRY(launch_begin(b, s->fp32, s->sm_count * 4, s->stream));
     s->launches++;
     s->begun = true;

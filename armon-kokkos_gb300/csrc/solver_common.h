@@ -97,7 +97,9 @@ void set_tile_axis(AxisGeom<T>& g, bool rows, int halo, int sms, int slots, int 
     const int spread = (int)std::max<int64_t>(1, (int64_t)g.nlines * segs / sms);
     g.tile_lines = std::max(1, std::min({rows ? fit : std::min(fit, want), g.nlines, spread}));
     g.tile_groups = (g.nlines + g.tile_lines - 1) / g.tile_lines;
-    g.tile_scan = rows ? g.tile_lines == 1 : g.tile_lines * kTileUnit <= 32 && len <= 56;
+    // worth a scan when a block has several tiles; the walls' positions may not overlap
+    g.tile_scan = (rows ? g.tile_lines == 1 : g.tile_lines * kTileUnit <= 32 && len <= 56) && g.n >= 32 &&
+                  (int64_t)segs * g.tile_groups >= 3 * (int64_t)slots;
     if (!rows && g.tile_scan)       // a large unit of columns lies in one segment
         g.tile_groups = (g.tile_groups + kTileUnit - 1) / kTileUnit * kTileUnit;
     const int64_t tiles = (int64_t)segs * g.tile_groups;
@@ -214,6 +216,7 @@ int make_sweep_args(const armon_params& p, int npass, int block, int sms, const 
     a.partials = partials;
     a.faces = nullptr;
     a.face_stride = 0;
+    a.hints = nullptr;
     return std::max(a.geom[0].blocks, a.geom[1].blocks);
 }
 

@@ -202,6 +202,14 @@ struct AxisGeom {
     int32_t tile_scan;    // units may be scanned for kept states (one row, or up to 32 columns, per unit)
 };
 
+// States that uniform regions of a domain probably hold (sweep_tile.cuh), per state buffer set:
+// rho, umat, vmat, Emat.
+template <class T>
+struct TileHints {
+    T v[2][2][4];
+    int32_t valid[2][2];
+};
+
 template <class T>
 struct SweepArgs {
     AxisGeom<T> geom[2];              // X, Y
@@ -221,6 +229,7 @@ struct SweepArgs {
     double* partials;                 // 2 doubles per block (dt reduction)
     T* faces;                         // split passes: u*, p*, p* u* per face (sweep_split.cuh)
     int64_t face_stride;              // values per face array
+    TileHints<T>* hints;              // tile passes
 };
 
 // ---- Exact reuse over runs of identical inputs (SweepArgs::reuse) ----

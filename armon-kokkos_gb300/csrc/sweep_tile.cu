@@ -1,5 +1,6 @@
 // sweep_tile.cu -- the tile form of the axis pass (sweep_tile.cuh) for both storage types.
 // Built with --fmad=false and IEEE division / square root, like the marches.
+#define ARMON_SFP_CALLS
 #include "launch.h"
 #include "sweep_tile.cuh"
 

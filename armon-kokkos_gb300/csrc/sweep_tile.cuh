@@ -31,6 +31,10 @@
 // consecutive chunks) in a list.  The block computes the list packed, several stretches side by side
 // in its threads, so that a thin front costs its own positions and not whole tiles.  A unit without
 // a uniform chunk is computed as tiles, and a block that keeps no state does not scan.
+// The results of the states a pass keeps are what its uniform regions hold next, so they are left as
+// hints: the next pass's blocks start by evaluating them (a window of equal cells, and the positions
+// next to either wall), and so know the resting regions, walls included, from their first unit.
+// A hint only proposes a state; cells take its results when they equal it bit for bit.
 #pragma once
 
 #include "sweep.cuh"
@@ -50,8 +54,9 @@ constexpr int kTileList = 512;        // stretches the list can hold (at most 12
 #endif
 template <class T> constexpr int tile_min_blocks() { return sizeof(T) == 8 ? ARMON_TILE_MIN_BLOCKS : ARMON_TILE_MIN_BLOCKS_F32; }
 
-// A kept state: the cell, its p and c, and the results of a position inside a run of it.
-enum : int { kRunRho, kRunUa, kRunUo, kRunE, kRunP, kRunC, kRunOut, kRunValues = kRunOut + 4 };
+// A kept state: the cell, its p and c, the results of a position inside a run of it, and the results of
+// the H <= 4 positions next to a wall (low side, high side) when the run reaches it.
+enum : int { kRunRho, kRunUa, kRunUo, kRunE, kRunP, kRunC, kRunOut, kRunWall = kRunOut + 4, kRunValues = kRunWall + 32 };
 
 // Consecutive owned positions of a line waiting to be computed.
 struct Stretch {
@@ -78,8 +83,9 @@ struct TileShared {
     uint32_t head;
     uint32_t tail[2];                 // [unit parity]
     int uniform[2];                   // [unit parity]: the unit holds a uniform chunk
-    int valid[2];
+    int valid[2];                     // bit 0: the state is kept; bit 1: with its walls
     int turn;                         // the kept state to replace next
+    int claims;                       // states recorded so far
     int next[2];                      // [unit parity]: the block's next unit
 };
 
@@ -98,8 +104,11 @@ struct TilePass {
     bool last = false, pcg = false;
     int tile_q = 0, tile_l = 0;       // the thread's position and line in a tile
     int parity = 0;
+    bool hints = false;               // the hinted states are still to be evaluated
+    uint32_t counted = 0;             // kept states whose speeds this thread has added (a bit each)
 
     struct Spot {                     // the thread's place
+        int hint;                     // the hinted state the thread stands for, -1 for a cell
         int q, t, width;              // position in the stretch (halo included), along the axis; positions of the stretch
         int64_t base;                 // index of position 0 of the line
         bool in;
@@ -132,6 +141,8 @@ struct TilePass {
             tile_q = tid / g.tile_lines;
             tile_l = tid - tile_q * g.tile_lines;
         }
+        hints = A.reuse && g.tile_scan && A.sw >= H &&
+                (__ldcg(&A.hints->valid[src][0]) | __ldcg(&A.hints->valid[src][1])) != 0;
         return true;
     }
 
@@ -148,6 +159,7 @@ struct TilePass {
         place(g, tile, seg, grp);
         const int a0 = seg * g.tile_len;
         Spot p;
+        p.hint = -1;
         p.q = tile_q;
         p.width = min(g.n, a0 + g.tile_len) - a0 + 2 * H;
         p.t = a0 - H + tile_q;
@@ -216,12 +228,16 @@ struct TilePass {
             if (threadIdx.x == 0) {
                 if (fetch) sh.next[parity] = after();
                 sh.tail[parity] = sh.tail[parity ^ 1];
+                sh.uniform[parity ^ 1] = 0;     // read before the last barrier, set after the next
             }
-            const bool v0 = sh.valid[0] != 0, v1 = sh.valid[1] != 0;
+            const int v0 = sh.valid[0], v1 = sh.valid[1], claims = sh.claims;
+            int seen = claims;
             // the same for every thread: a barrier follows each of their writes
-            const bool scan = g.tile_scan && (v0 || v1);
+            bool evaluate = hints;
+            hints = false;
+            const bool scan = g.tile_scan && (v0 | v1) && !evaluate;
             // a block that keeps no state yet takes a tile at a time, to scan the rest once it does
-            const int nk = scan || !g.tile_scan ? end - tile : 1;
+            int nk = evaluate ? 0 : scan || !g.tile_scan ? end - tile : 1;
             int k = 0;
             if (scan) {
                 if (axis == 0) scan_rows(g, tile, nk, v0, v1);
@@ -234,23 +250,29 @@ struct TilePass {
                 }
             }
             __syncthreads();
-            if (threadIdx.x == 0) sh.uniform[parity ^ 1] = 0;    // for the next scan
             if (fetch) next = sh.next[parity];
             fetch = false;
-            const bool all = next >= total && tile + nk >= end;
-            // the tiles, or the list's stretches, packed
+            const bool all = next >= total && tile + nk >= end && !evaluate;
+            // the hinted states, the tiles, or the list's stretches, packed
             for (;;) {
                 Spot p;
-                int ds = 1, centre;
-                if (k < nk) {
+                int ds = 1, centre = -1;
+                if (evaluate) {
+                    p = hint_spot(g);
+                } else if (k < nk) {
+                    if (scan && seen != claims) {   // a state more is kept: scan the rest again
+                        nk = k;
+                        continue;
+                    }
                     p = tile_spot(g, tile + k);
                     if (axis != 0) ds = g.tile_lines;
                     centre = (p.width / 2) * ds;      // the middle of the tile's first line
                     k++;
-                } else if (!pack(all, p, centre)) {
+                } else if (nk == 0 || !pack(all && tile + nk >= end, p, centre)) {
                     break;
                 }
-                compute(g, p, ds, centre);
+                seen = compute(g, p, ds, centre);
+                evaluate = false;
             }
             tile += nk;
         }
@@ -258,11 +280,11 @@ struct TilePass {
     }
 
     // ---- scan ----
-    // Ghosts never match (their mirrored velocities differ from a state at rest by the sign of zero), so
-    // the chunks next to a wall are computed.
+    // Ghosts (whose mirrored velocities differ from a state at rest by the sign of zero) match a state
+    // that is kept with its walls' results.
     // Rows: warp w takes the unit's tile w, its positions 32 at a time; match[state][w][i] is the ballot
     // of positions 32 i .. 32 i + 31 of the tile (positions past its end count as matching).
-    __device__ __forceinline__ void scan_rows(const AxisGeom<T>& g, int tile0, int nk, bool v0, bool v1)
+    __device__ __forceinline__ void scan_rows(const AxisGeom<T>& g, int tile0, int nk, int v0, int v1)
     {
         const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
         if (w >= nk) return;
@@ -286,8 +308,8 @@ struct TilePass {
             for (int i = 0; i < kBatch; i++) {
                 const int q = 32 * (i0 + i) + lane, t = a0 - H + q;
                 const bool out = q >= width, real = t >= 0 && t < g.n;
-                const uint32_t b0 = __ballot_sync(0xffffffffu, out || (v0 && real && same_as_kept(c[i], 0)));
-                const uint32_t b1 = __ballot_sync(0xffffffffu, out || (v1 && real && same_as_kept(c[i], 1)));
+                const uint32_t b0 = __ballot_sync(0xffffffffu, out || (real ? v0 && same_as_kept(c[i], 0) : v0 > 1));
+                const uint32_t b1 = __ballot_sync(0xffffffffu, out || (real ? v1 && same_as_kept(c[i], 1) : v1 > 1));
                 if (lane == 0) {
                     sh.match[parity][0][w][i0 + i] = b0;
                     sh.match[parity][1][w][i0 + i] = b1;
@@ -327,8 +349,8 @@ struct TilePass {
         const int64_t base = A.origin + (int64_t)grp * g.lstride + a0;
         for (int o = lane; o < len; o += 32) {
             const int j = o >> 3;
-            if ((idle0 >> j) & 1u) store_kept(base + o, 0);
-            else if ((idle1 >> j) & 1u) store_kept(base + o, 1);
+            if ((idle0 >> j) & 1u) store_kept(g, base + o, a0 + o, 0);
+            else if ((idle1 >> j) & 1u) store_kept(g, base + o, a0 + o, 1);
         }
     }
     // Appends the runs of a line's chunks in `todo` (bit j: chunk j, at a0 + 8 j) to the list; runs one
@@ -346,24 +368,53 @@ struct TilePass {
         const uint32_t at = atomicAdd(&sh.tail[parity], 1u);
         sh.list[at % kTileList] = Stretch{line, ((a0 + 8 * j) << 8) | cells};
     }
-    __device__ __forceinline__ void store_kept(int64_t i, int e)
+    // The results of position t, at index i, of a run of kept state e.
+    __device__ __forceinline__ void store_kept(const AxisGeom<T>& g, int64_t i, int t, int e)
     {
         const T* kv = sh.kept[e];
+        const bool wall = t < H || t >= g.n - H;
+        const T* o = kv + (!wall ? (int)kRunOut : t < H ? kRunWall + 4 * t : kRunWall + 16 + 4 * (t - (g.n - H)));
         T* const* out = A.buf[src ^ 1];
-        out[0][i] = kv[kRunOut];
-        out[1 + axis][i] = kv[kRunOut + 1];
-        out[2 - axis][i] = kv[kRunOut + 2];
-        out[3][i] = kv[kRunOut + 3];
+        out[0][i] = o[0];
+        out[1 + axis][i] = o[1];
+        out[2 - axis][i] = o[2];
+        out[3][i] = o[3];
         if (pcg) {
             A.pmat[i] = kv[kRunP];
             A.cmat[i] = kv[kRunC];
             A.gmat[i] = (1 + A.gamma) / 2;
         }
+        if (last && (wall || !((counted >> e) & 1u))) {
+            if (!wall) counted |= 1u << e;
+            add_dt(o, kv[kRunC]);
+        }
+    }
+    // dt_CFL of the state after this pass, with c from this pass's EOS
+    __device__ __forceinline__ void add_dt(const T* o, T c)
+    {
+        if (axis == 0) sh.acc[threadIdx.x].add(o[1], o[2], c);
+        else sh.acc[threadIdx.x].add(o[2], o[1], c);
+    }
+    // The evaluation of the hinted states: per state, threads for a position inside a run of it (a
+    // window of 2 H + 1 cells) and for the H positions next to either wall.
+    __device__ __forceinline__ Spot hint_spot(const AxisGeom<T>& g) const
+    {
+        constexpr int kPlain = 2 * H + 1, kSide = 3 * H, kAll = kPlain + 2 * kSide;
+        const int tid = threadIdx.x;
+        const int r = tid % kAll;
+        Spot p;
+        p.hint = tid / kAll;
+        p.in = p.hint < 2 && __ldcg(&A.hints->valid[src][min(p.hint, 1)]);
+        p.base = 0;
+        if (r < kPlain) { p.q = r; p.width = kPlain; p.t = g.n / 2; }
+        else if (r < kPlain + kSide) { p.q = r - kPlain; p.width = kSide; p.t = p.q - H; }
+        else { p.q = r - kPlain - kSide; p.width = kSide; p.t = g.n - 2 * H + p.q; }
+        return p;
     }
     // Columns: the unit's tiles are columns line0 .. of one segment, a lane each; warp w takes positions
     // 8 w .. 8 w + 7 of the segment (halo included), and match[state][0][w] has bit c set when they all
     // match in column c.  Chunk j of a column is uniform when words j and j + 1 have its bit.
-    __device__ __forceinline__ void scan_columns(const AxisGeom<T>& g, int tile0, int nk, bool v0, bool v1)
+    __device__ __forceinline__ void scan_columns(const AxisGeom<T>& g, int tile0, int nk, int v0, int v1)
     {
         const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
         int seg, grp;
@@ -374,7 +425,7 @@ struct TilePass {
         const int width = min(g.n, a0 + g.tile_len) - a0 + 2 * H;
         const int64_t base = A.origin + (int64_t)line * g.lstride;
         constexpr int kBatch = sizeof(T) == 8 ? 4 : 8;
-        bool m0 = v0, m1 = v1;
+        bool m0 = v0 != 0, m1 = v1 != 0;
         if (col) {
 #pragma unroll 1
             for (int i0 = 0; i0 < 8; i0 += kBatch) {
@@ -389,8 +440,8 @@ struct TilePass {
                 for (int i = 0; i < kBatch; i++) {
                     const int q = 8 * w + i0 + i, t = a0 - H + q;
                     const bool out = q >= width, real = t >= 0 && t < g.n;
-                    m0 = m0 && (out || (real && same_as_kept(c[i], 0)));
-                    m1 = m1 && (out || (real && same_as_kept(c[i], 1)));
+                    m0 = m0 && (out || (real ? same_as_kept(c[i], 0) : v0 > 1));
+                    m1 = m1 && (out || (real ? same_as_kept(c[i], 1) : v1 > 1));
                 }
             }
         }
@@ -423,7 +474,7 @@ struct TilePass {
             const int e = !col ? -1 : ((M0[w] & M0[w + 1]) >> lane) & 1u ? 0 : ((M1[w] & M1[w + 1]) >> lane) & 1u ? 1 : -1;
             if (e >= 0) {
                 const int end = min(8 * w + 8, len);
-                for (int o = 8 * w; o < end; o++) store_kept(A.origin + (int64_t)line * g.lstride + (int64_t)(a0 + o) * g.s, e);
+                for (int o = 8 * w; o < end; o++) store_kept(g, A.origin + (int64_t)line * g.lstride + (int64_t)(a0 + o) * g.s, a0 + o, e);
             }
         } else if (col) {
             // the last warp lists the others' chunks, a lane per column
@@ -467,6 +518,7 @@ struct TilePass {
         }
         const int line = __shfl_sync(0xffffffffu, s.line, k);
         const int sl = __shfl_sync(0xffffffffu, s.start_len, k);
+        p.hint = -1;
         p.q = tid - __shfl_sync(0xffffffffu, sum - need, k);
         p.width = (sl & 255) + 2 * H;
         p.t = (sl >> 8) - H + p.q;
@@ -500,21 +552,23 @@ struct TilePass {
             same = same_state(o, u);
         }
         if (!__all_sync(0xffffffffu, same)) return -1;
-        const bool v0 = sh.valid[0] != 0, v1 = sh.valid[1] != 0;
+        const int v0 = sh.valid[0], v1 = sh.valid[1];
         if ((v0 && same_as_kept(u, 0)) || (v1 && same_as_kept(u, 1))) return -1;
         const int s = !v0 ? 0 : !v1 ? 1 : sh.turn;
         __syncwarp();
         if (lane == 0) {
             sh.valid[s] = 0;
             sh.turn = s ^ 1;
+            sh.claims++;
         }
         __syncwarp();
         return s;
     }
 
     // The stages at the thread's position; ds threads between neighbouring positions.  The centre
-    // thread records its state when it can.
-    __device__ __forceinline__ void compute(const AxisGeom<T>& g, const Spot& p, const int ds, const int centre)
+    // thread records its state when it can.  Returns sh.claims as every thread of the block sees it: read
+    // between the barrier that follows this call's claim and the ones before the next call's.
+    __device__ __forceinline__ int compute(const AxisGeom<T>& g, const Spot& p, const int ds, const int centre)
     {
         const int tid = threadIdx.x;
         const T dx = g.dx;
@@ -532,14 +586,22 @@ struct TilePass {
             int m, side;
             const bool stale = source(g.n, p.t, m, side);
             const int64_t i = p.base + (int64_t)m * g.s;
-            load(i, c);
+            if (p.hint >= 0) {
+                const T* v = A.hints->v[src][p.hint];
+                c.rho = __ldcg(v);
+                c.ua = __ldcg(v + 1 + axis);
+                c.uo = __ldcg(v + 2 - axis);
+                c.E = __ldcg(v + 3);
+            } else {
+                load(i, c);
+            }
             mirror(g, c, side);
             if (stale) {
                 c.p = A.pmat[i];
                 c.c = A.cmat[i];
             } else {
                 eos(c, A.gamma, A.gamma - 1);
-                if (pcg && own) {
+                if (pcg && own && p.hint < 0) {
                     A.pmat[i] = c.p;
                     A.cmat[i] = c.c;
                     A.gmat[i] = (1 + A.gamma) / 2;
@@ -555,9 +617,13 @@ struct TilePass {
             ARMON_X(13) = c.dm;
             sh.c[tid] = c.c;
         }
-        if (A.reuse && g.tile_scan && (tid >> 5) == (centre >> 5)) {
-            rec = claim_slot(g, p, c, centre);
-            if (tid != centre) rec = -1;
+        if (A.reuse && g.tile_scan) {
+            if (p.hint >= 0) {
+                if (on && q == H && width == 2 * H + 1) rec = p.hint;
+            } else if ((tid >> 5) == (centre >> 5)) {
+                rec = claim_slot(g, p, c, centre);
+                if (tid != centre) rec = -1;
+            }
             if (rec >= 0) {
                 T* const rv = sh.kept[rec];
                 rv[kRunRho] = c.rho; rv[kRunUa] = c.ua; rv[kRunUo] = c.uo; rv[kRunE] = c.E;
@@ -565,6 +631,7 @@ struct TilePass {
             }
         }
         __syncthreads();
+        const int claims = sh.claims;
 
         // ---- Godunov face q (between positions q - 1 and q) ----
         God<T> G{};
@@ -668,7 +735,7 @@ struct TilePass {
             ARMON_X(2) = a.ro;
             ARMON_X(14) = a.rE;
         }
-        if (rec >= 0) sh.valid[rec] = 1;    // its results follow; they are read after the next unit's first barrier
+        if (rec >= 0) sh.valid[rec] = p.hint >= 0 ? 3 : 1;    // its results follow; they are read after the next unit's first barrier
         __syncthreads();
 
         // ---- projection of cell q (src/kernels/euler_projection.cpp:36-46) ----
@@ -683,25 +750,34 @@ struct TilePass {
             o[1] = qdiv_at<8>(ra, inv_rho);
             o[2] = qdiv_at<8>(ro, inv_rho);
             o[3] = qdiv_at<8>(rE, inv_rho);
-            const int64_t i = p.base + (int64_t)p.t * g.s;
-            T* const* out = A.buf[src ^ 1];
-            out[0][i] = o[0];
-            out[1 + axis][i] = o[1];
-            out[2 - axis][i] = o[2];
-            out[3][i] = o[3];
-            if (last) {
-                // dt_CFL of the state after this pass, with c from this pass's EOS; a kept state was
-                // recorded by a thread that adds it here
-                if (axis == 0) sh.acc[tid].add(o[1], o[2], sh.c[tid]);
-                else sh.acc[tid].add(o[2], o[1], sh.c[tid]);
+            if (p.hint < 0) {
+                const int64_t i = p.base + (int64_t)p.t * g.s;
+                T* const* out = A.buf[src ^ 1];
+                out[0][i] = o[0];
+                out[1 + axis][i] = o[1];
+                out[2 - axis][i] = o[2];
+                out[3][i] = o[3];
+                if (last) add_dt(o, sh.c[tid]);
+            } else if (rec < 0) {
+                T* const wv = sh.kept[p.hint] + (p.t < H ? kRunWall + 4 * p.t : kRunWall + 16 + 4 * (p.t - (g.n - H)));
+                wv[0] = o[0]; wv[1] = o[1]; wv[2] = o[2]; wv[3] = o[3];
             }
             if (rec >= 0) {
                 T* const rv = sh.kept[rec];
                 rv[kRunOut] = o[0]; rv[kRunOut + 1] = o[1]; rv[kRunOut + 2] = o[2]; rv[kRunOut + 3] = o[3];
+                // a run of this state is one of its results for the next pass
+                TileHints<T>* h = A.hints;
+                T* v = h->v[src ^ 1][rec];
+                v[0] = o[0];
+                v[1 + axis] = o[1];
+                v[2 - axis] = o[2];
+                v[3] = o[3];
+                h->valid[src ^ 1][rec] = 1;
             }
         }
 #undef ARMON_X
 #undef ARMON_AT
+        return claims;
     }
 };
 
@@ -774,12 +850,19 @@ __device__ __forceinline__ bool tile_arrive(TileCtl* ctl)
     return is_last != 0;
 }
 
+// The hints this pass has used are written again by the next.
+template <class T>
+__device__ __forceinline__ void tile_clear_hints(const SweepArgs<T>& A, int src)
+{
+    A.hints->valid[src][0] = A.hints->valid[src][1] = 0;
+}
+
 template <class T>
 __device__ __forceinline__ void tile_forget(TileShared<T>& sh)
 {
     if (threadIdx.x == 0) {
         sh.valid[0] = sh.valid[1] = 0;
-        sh.turn = 0;
+        sh.turn = sh.claims = 0;
         sh.head = sh.tail[0] = sh.tail[1] = 0;
         sh.uniform[0] = sh.uniform[1] = 0;
     }
@@ -794,7 +877,8 @@ tile_kernel(const __grid_constant__ SweepArgs<T> A, TileCtl* ctl, int last)
     TilePass<T, SCHEME, PROJ> P(A, sh);
     tile_forget(sh);
     sh.acc[threadIdx.x].init();
-    if (P.start(A.pass, last != 0, blockIdx.x == 0 && threadIdx.x == 0)) {
+    const bool ran = P.start(A.pass, last != 0, blockIdx.x == 0 && threadIdx.x == 0);
+    if (ran) {
         const int total = A.geom[P.axis].tile_units;
         __syncthreads();
         int u = blockIdx.x;
@@ -805,7 +889,10 @@ tile_kernel(const __grid_constant__ SweepArgs<T> A, TileCtl* ctl, int last)
         }
         if (last) tile_flush(sh, A.state);
     }
-    if (tile_arrive(ctl) && last && threadIdx.x == 0) tile_commit(A.state, A.cfg);
+    if (tile_arrive(ctl) && threadIdx.x == 0) {
+        if (ran) tile_clear_hints(A, P.src);
+        if (last) tile_commit(A.state, A.cfg);
+    }
 }
 
 }  // namespace armon
