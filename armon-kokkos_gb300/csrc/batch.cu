@@ -54,6 +54,7 @@ struct Dom {
     int64_t npartials = 0;        // pairs
     void* faces = nullptr;        // split passes: 3 face arrays of face_values(p) values
     int seg_len = 0;
+    bool eos_stale = false;       // tile passes have run since p, c, g were stored
 };
 
 // values per face array of a split pass (sweep_split.cuh): the larger axis's (n + 5) * nlines
@@ -108,6 +109,12 @@ struct armon_batch {
     cudaGraphExec_t graph = nullptr;
     int64_t bytes = 0;
     int64_t launches = 0;
+    bool tile = true;             // passes in the tile form (sweep_tile.cuh), unless a domain fixes its segments
+    bool tiled = true;            // the current table's form
+    int* d_units = nullptr;       // tile form: units of each domain
+    uint32_t* d_tickets = nullptr;
+    TileCtl* d_ctl = nullptr;
+    TileHints<double>* d_hints = nullptr;   // per slot
     bool split = true;            // passes as a face launch and a cell launch (sweep_split.cuh)
     bool ordered = true;          // longest-first dispatch of each pass's blocks
     uint32_t* d_order = nullptr;  // per pass (and per half of a split pass) order_cap block indices
@@ -208,12 +215,66 @@ std::vector<std::array<int, 2>> schedule_segments(const armon_batch* b)
 // order / cost arrays: one per pass of a cycle, and one more per pass for the face halves
 int order_arrays(const armon_batch* b) { return b->npass * (b->split ? 2 : 1); }
 
+// The launch table of tile passes.  The resident blocks are shared out to the domains in proportion to
+// their cells (a domain of less than half a block's share gets none and is joined by blocks that
+// finish theirs); a domain's tiles are cut as if it had that share of the GPU to itself.
+template <class T>
+int rebuild_tiles(armon_batch* b)
+{
+    const size_t nd = b->table.size();
+    if (b->blocks_per_sm == 0) b->blocks_per_sm = sweep_tile_batch_blocks_per_sm(b->fp32, b->scheme, b->proj);
+    const int slots = b->sm_count * b->blocks_per_sm;
+    double total = 0;
+    for (int i : b->table) total += double(b->doms[i].p.nx) * b->doms[i].p.ny;
+    std::vector<SweepArgs<T>> args(nd);
+    std::vector<int> first(nd + 1, 0), units(nd, 0);
+    double seen = 0;
+    int64_t all = 0;
+    for (size_t k = 0; k < nd; k++) {
+        Dom& d = b->doms[b->table[k]];
+        const int whole[2] = {d.p.nx, d.p.ny};
+        make_sweep_args<T>(d.p, b->npass, b->o.block_lines, b->sm_count, whole, buffers<T>(d), b->d_states + b->table[k],
+                           d.partials, -1, b->o.reuse >= 0 ? 1 : 0, args[k]);
+        args[k].hints = reinterpret_cast<TileHints<T>*>(b->d_hints + b->table[k]);
+        const double share = double(d.p.nx) * d.p.ny / total;
+        for (int axis = 0; axis < 2; axis++) {
+            set_tile_axis(args[k].geom[axis], axis == 0, stencil_reach(&d.p),
+                          std::max(1, (int)std::lround(b->sm_count * share)),
+                          std::max(1, (int)std::lround(slots * share)), kTileYLines);
+            units[k] = std::max(units[k], args[k].geom[axis].tile_units);
+        }
+        seen += share;
+        first[k + 1] = std::min((int)std::lround(slots * seen), first[k] + units[k]);
+        all += units[k];
+    }
+    // at least one block, and no more than there are units
+    if (first[nd] == 0)
+        for (size_t k = 1; k <= nd; k++) first[k] = 1;
+    b->total_blocks = first[nd];
+    CUDA_TRY(cudaMemcpyAsync(b->d_args, args.data(), nd * sizeof(SweepArgs<T>), cudaMemcpyHostToDevice, b->stream));
+    CUDA_TRY(cudaMemcpyAsync(b->d_offsets, first.data(), (nd + 1) * sizeof(int), cudaMemcpyHostToDevice, b->stream));
+    CUDA_TRY(cudaMemcpyAsync(b->d_units, units.data(), nd * sizeof(int), cudaMemcpyHostToDevice, b->stream));
+    CUDA_TRY(cudaMemsetAsync(b->d_tickets, 0, nd * sizeof(uint32_t), b->stream));
+    CUDA_TRY(cudaStreamSynchronize(b->stream));   // the host vectors go out of scope
+    return ARMON_OK;
+}
+
 template <class T>
 int rebuild_t(armon_batch* b)
 {
     b->table.clear();
     for (int i = 0; i < (int)b->doms.size(); i++)
         if (b->doms[i].used && !b->doms[i].done) b->table.push_back(i);
+    bool tiled = b->tile;
+    for (int i : b->table) tiled = tiled && b->doms[i].seg_len <= 0;
+    if (tiled != b->tiled) b->blocks_per_sm = 0;
+    b->tiled = tiled;
+    if (b->graph) {
+        cudaGraphExecDestroy(b->graph);
+        b->graph = nullptr;
+    }
+    b->dirty = false;
+    if (tiled) return b->table.empty() ? ARMON_OK : rebuild_tiles<T>(b);
     if (b->blocks_per_sm == 0 && !b->table.empty())
         b->blocks_per_sm = b->split ? sweep_batch_split_blocks_per_sm(b->fp32, b->scheme, b->proj, b->o.block_lines)
                                     : sweep_batch_blocks_per_sm(b->fp32, b->scheme, b->proj, b->o.block_lines);
@@ -260,11 +321,6 @@ int rebuild_t(armon_batch* b)
                                  b->stream));
         CUDA_TRY(cudaStreamSynchronize(b->stream));   // the host vectors go out of scope
     }
-    if (b->graph) {
-        cudaGraphExecDestroy(b->graph);
-        b->graph = nullptr;
-    }
-    b->dirty = false;
     return ARMON_OK;
 }
 
@@ -277,7 +333,7 @@ int64_t table_cells(const armon_batch* b)
     return c;
 }
 
-bool schedule_fixed(const armon_batch* b) { return b->o.waves > 0 || b->o.seg_len > 0; }
+bool schedule_fixed(const armon_batch* b) { return b->tiled || b->o.waves > 0 || b->o.seg_len > 0; }
 
 // Online autotuning of the schedule: each candidate number of waves is timed with CUDA events over
 // one graph batch of real cycles (results do not depend on the segments, so nothing is wasted);
@@ -326,6 +382,18 @@ int enqueue_direct(armon_batch* b, int n)
     for (int c = 0; c < n; c++) {
         for (int k = 0; k < b->npass; k++) {
             bool last = k == b->npass - 1;
+            if (b->tiled) {
+                const cudaError_t e =
+                    b->fp32 ? launch_sweep_tile_batch((const SweepArgs<float>*)b->d_args, b->d_offsets, b->d_units,
+                                                      b->d_tickets, nd, k, b->d_ctl, b->scheme, b->proj, last,
+                                                      b->total_blocks, b->stream)
+                            : launch_sweep_tile_batch((const SweepArgs<double>*)b->d_args, b->d_offsets, b->d_units,
+                                                      b->d_tickets, nd, k, b->d_ctl, b->scheme, b->proj, last,
+                                                      b->total_blocks, b->stream);
+                if (e != cudaSuccess) return cuda_fail(e, "batch tile launch");
+                b->launches++;
+                continue;
+            }
             BatchOrder ord{nullptr, nullptr}, ford{nullptr, nullptr};
             if (b->ordered) {
                 ord.order = b->d_order + (size_t)k * b->order_cap;
@@ -349,7 +417,7 @@ int enqueue_direct(armon_batch* b, int n)
             if (e != cudaSuccess) return cuda_fail(e, "batch sweep launch");
             b->launches += b->split ? 2 : 1;
         }
-        if (b->ordered) {
+        if (b->ordered && !b->tiled) {
             UnitCounts counts;
             for (int a = 0; a < kMaxOrderArrays; a++) counts.n[a] = b->total_blocks;
             order_units_kernel<<<order_arrays(b), 1024, 0, b->stream>>>(b->d_cost, b->d_order, b->order_cap, counts);
@@ -373,6 +441,8 @@ int enqueue(armon_batch* b, int n)
         if (rc != ARMON_OK) return rc;
     }
     if (b->table.empty() || n <= 0) return ARMON_OK;
+    if (b->tiled)
+        for (int i : b->table) b->doms[i].eos_stale = true;
     const int gc = b->o.cycles_per_graph;
     if (gc > 0 && n >= gc) {
         if (!b->graph) {
@@ -397,7 +467,7 @@ int enqueue(armon_batch* b, int n)
                 b->tune.launched = true;
                 b->tune.work = double(table_cells(b)) * gc;
             }
-            b->launches += (int64_t)gc * (b->npass * (b->split ? 2 : 1) + (b->ordered ? 1 : 0));
+            b->launches += (int64_t)gc * (b->tiled ? b->npass : b->npass * (b->split ? 2 : 1) + (b->ordered ? 1 : 0));
             n -= gc;
         }
     }
@@ -458,6 +528,8 @@ int armon_batch_create(const armon_batch_opts* opts, void* stream, armon_batch**
     b->ordered = b->o.unit_order >= 0;
     b->split = b->o.split_pass > 0 || (b->o.split_pass == 0 && split_default(b->o.precision));
     if (b->o.waves > 0) b->waves = b->o.waves;
+    // the tile form unless the caller asks for something of the marches'
+    b->tile = b->tiled = b->o.split_pass == 0 && b->o.seg_len <= 0 && b->o.waves <= 0 && b->o.block_lines == 128;
     int dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&b->sm_count, cudaDevAttrMultiProcessorCount, dev);
@@ -486,6 +558,11 @@ int armon_batch_create(const armon_batch_opts* opts, void* stream, armon_batch**
     if (e == cudaSuccess) e = cudaMallocHost(&b->h_states, sizeof(StepState) * kMaxDomains);
     if (e == cudaSuccess) e = cudaMalloc(&b->d_args, sizeof(SweepArgs<double>) * kMaxDomains);
     if (e == cudaSuccess) e = cudaMalloc(&b->d_offsets, sizeof(int) * (kMaxDomains + 1));
+    if (e == cudaSuccess) e = cudaMalloc(&b->d_units, sizeof(int) * kMaxDomains);
+    if (e == cudaSuccess) e = cudaMalloc(&b->d_tickets, sizeof(uint32_t) * kMaxDomains + sizeof(TileCtl));
+    if (e == cudaSuccess) e = cudaMemset(b->d_tickets, 0, sizeof(uint32_t) * kMaxDomains + sizeof(TileCtl));
+    if (e == cudaSuccess) e = cudaMalloc(&b->d_hints, sizeof(TileHints<double>) * kMaxDomains);
+    b->d_ctl = reinterpret_cast<TileCtl*>(b->d_tickets + kMaxDomains);
     if (e != cudaSuccess) {
         armon_batch_destroy(b);
         return cuda_fail(e, "batch allocation");
@@ -508,6 +585,9 @@ void armon_batch_destroy(armon_batch* b)
     if (b->h_states) cudaFreeHost(b->h_states);
     if (b->d_args) cudaFree(b->d_args);
     if (b->d_offsets) cudaFree(b->d_offsets);
+    if (b->d_units) cudaFree(b->d_units);
+    if (b->d_tickets) cudaFree(b->d_tickets);
+    if (b->d_hints) cudaFree(b->d_hints);
     if (b->d_order) cudaFree(b->d_order);
     if (b->d_cost) cudaFree(b->d_cost);
     if (b->ev0) cudaEventDestroy(b->ev0);
@@ -612,6 +692,7 @@ int add_domain(armon_batch* b, const armon_params* p, const double* const init[4
     for (int k = 0; k < 4; k++)
         CUDA_TRY(cudaMemcpyAsync(dd.arr[4 + k], dd.arr[k], arr_bytes, cudaMemcpyDeviceToDevice, b->stream));
     CUDA_TRY(cudaMemsetAsync(b->d_states + slot, 0, sizeof(StepState), b->stream));
+    CUDA_TRY(cudaMemsetAsync(b->d_hints + slot, 0, sizeof(TileHints<double>), b->stream));
     BeginArgs ba{};
     ba.nx = p->nx; ba.ny = p->ny;
     ba.origin = (int64_t)p->nb_ghosts * p->row_length + p->nb_ghosts;
@@ -727,6 +808,22 @@ int armon_batch_download(armon_batch* b, int32_t id, int which, double* host)
     CUDA_TRY(cudaMemcpyAsync(&b->h_states[id], b->d_states + id, sizeof(StepState), cudaMemcpyDeviceToHost, b->stream));
     CUDA_TRY(cudaStreamSynchronize(b->stream));
     Dom& d = b->doms[id];
+    if (which >= 6 && d.eos_stale && b->h_states[id].cycle > 0) {
+        // tile passes store no p, c, g: those of the last pass's input, which the set the current state is
+        // not in still holds, are computed when they are read
+        const int in = 4 * (current_set(b, id) ^ 1);
+        BeginArgs ba{};
+        ba.nx = d.p.nx; ba.ny = d.p.ny;
+        ba.origin = (int64_t)d.p.nb_ghosts * d.p.row_length + d.p.nb_ghosts;
+        ba.row_length = d.p.row_length;
+        ba.gamma = 1.4;
+        ba.rho = d.arr[in]; ba.umat = d.arr[in + 1]; ba.vmat = d.arr[in + 2]; ba.Emat = d.arr[in + 3];
+        ba.pmat = d.arr[8]; ba.cmat = d.arr[9]; ba.gmat = d.arr[10];
+        ba.eos_only = 1;
+        CUDA_TRY(launch_begin(ba, b->fp32, 152 * 4, b->stream));
+        b->launches++;
+        d.eos_stale = false;
+    }
     int k = which <= 5 ? current_set(b, id) * 4 + (which - 2) : 8 + (which - 6);
     size_t n = (size_t)d.p.nb_cells;
     if (!b->fp32) {

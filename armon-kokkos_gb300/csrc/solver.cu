@@ -99,7 +99,6 @@ int cuda_fail(cudaError_t e, const char* what)
         if (e_ != cudaSuccess) return cuda_fail(e_, #expr);       \
     } while (0)
 
-constexpr int kTileYLines = 4;
 // the step state, then the tile launches' counters and hints
 constexpr size_t kStateBytes = sizeof(StepState) + sizeof(TileCtl) + sizeof(TileHints<double>);
 

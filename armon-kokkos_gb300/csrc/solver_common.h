@@ -73,8 +73,9 @@ inline AxisTiling choose_segments(int n, int nlines, int block, int halo, int sm
     return axis_tiling(n, nlines, block, best_seg);
 }
 
-// Threads of a tile (sweep_tile.cuh).
+// Threads of a tile (sweep_tile.cuh), and the columns of a Y tile: four (FP64) are a sector.
 constexpr int kTileBlock = 256;
+constexpr int kTileYLines = 4;
 
 // The tiles of one axis.  A tile is `lines` lines by width = len + 2 halo positions, at most kTileBlock
 // threads.  Along rows (X) the positions are consecutive in memory, so a tile is as long as the block

@@ -36,6 +36,35 @@ int tile_blocks_t(int scheme, int proj)
     return (e == cudaSuccess && n > 0) ? n : 1;
 }
 
+template <class T>
+cudaError_t launch_tile_batch_t(const SweepArgs<T>* doms, const int* first, const int* units, uint32_t* tickets, int ndom,
+                                int pass, TileCtl* ctl, int scheme, int proj, bool last, int grid, cudaStream_t st)
+{
+#define ARMON_TB(S, P) \
+    tile_batch_kernel<T, S, P><<<grid, kTileThreads, 0, st>>>(doms, first, units, tickets, ndom, pass, ctl, last ? 1 : 0)
+    if (scheme == 1) {
+        if (proj == 2) ARMON_TB(1, 2); else ARMON_TB(1, 1);
+    } else {
+        if (proj == 2) ARMON_TB(0, 2); else ARMON_TB(0, 1);
+    }
+#undef ARMON_TB
+    return cudaGetLastError();
+}
+
+template <class T>
+int tile_batch_blocks_t(int scheme, int proj)
+{
+    int n = 0;
+    cudaError_t e;
+    if (scheme == 1)
+        e = proj == 2 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, tile_batch_kernel<T, 1, 2>, kTileThreads, 0)
+                      : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, tile_batch_kernel<T, 1, 1>, kTileThreads, 0);
+    else
+        e = proj == 2 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, tile_batch_kernel<T, 0, 2>, kTileThreads, 0)
+                      : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, tile_batch_kernel<T, 0, 1>, kTileThreads, 0);
+    return (e == cudaSuccess && n > 0) ? n : 1;
+}
+
 }  // namespace
 
 cudaError_t launch_sweep_tile(const SweepArgs<double>& a, TileCtl* ctl, int scheme, int proj, bool last, int grid,
@@ -48,6 +77,25 @@ cudaError_t launch_sweep_tile(const SweepArgs<float>& a, TileCtl* ctl, int schem
                               cudaStream_t st)
 {
     return launch_tile_t<float>(a, ctl, scheme, proj, last, grid, st);
+}
+
+cudaError_t launch_sweep_tile_batch(const SweepArgs<double>* doms, const int* first, const int* units, uint32_t* tickets,
+                                    int ndom, int pass, TileCtl* ctl, int scheme, int proj, bool last, int grid,
+                                    cudaStream_t st)
+{
+    return launch_tile_batch_t<double>(doms, first, units, tickets, ndom, pass, ctl, scheme, proj, last, grid, st);
+}
+
+cudaError_t launch_sweep_tile_batch(const SweepArgs<float>* doms, const int* first, const int* units, uint32_t* tickets,
+                                    int ndom, int pass, TileCtl* ctl, int scheme, int proj, bool last, int grid,
+                                    cudaStream_t st)
+{
+    return launch_tile_batch_t<float>(doms, first, units, tickets, ndom, pass, ctl, scheme, proj, last, grid, st);
+}
+
+int sweep_tile_batch_blocks_per_sm(bool fp32, int scheme, int proj)
+{
+    return fp32 ? tile_batch_blocks_t<float>(scheme, proj) : tile_batch_blocks_t<double>(scheme, proj);
 }
 
 int sweep_tile_blocks_per_sm(bool fp32, int scheme, int proj)

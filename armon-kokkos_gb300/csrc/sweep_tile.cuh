@@ -131,6 +131,7 @@ struct TilePass {
         dt = T(cd.current * factor);
         src = (int)(((int64_t)st.cycle * A.npass + pass + st.buf_base) & 1);
         last = last_pass;
+        counted = 0;
         pcg = A.write_eos > 0 || (last_pass && A.write_eos == 0);
         const AxisGeom<T>& g = A.geom[axis];
         const int tid = threadIdx.x;
@@ -220,10 +221,11 @@ struct TilePass {
     {
         const AxisGeom<T>& g = A.geom[axis];
         int tile = u < g.tile_big ? u * kTileUnit : g.tile_big * kTileUnit + (u - g.tile_big);
-        const int end = u < g.tile_big ? tile + kTileUnit : tile + 1;
+        // (a batch's domains have as many units as their larger axis: those past the axis's own are empty)
+        const int end = u < g.tile_big ? tile + kTileUnit : u < g.tile_units ? tile + 1 : tile;
         int next = total;
         bool fetch = true;
-        while (tile < end) {
+        do {
             parity ^= 1;
             if (threadIdx.x == 0) {
                 if (fetch) sh.next[parity] = after();
@@ -233,11 +235,12 @@ struct TilePass {
             const int v0 = sh.valid[0], v1 = sh.valid[1], claims = sh.claims;
             int seen = claims;
             // the same for every thread: a barrier follows each of their writes
+            const bool waiting = hints;      // only the hinted states this time
             bool evaluate = hints;
             hints = false;
-            const bool scan = g.tile_scan && (v0 | v1) && !evaluate;
+            const bool scan = g.tile_scan && (v0 | v1) && !evaluate && tile < end;
             // a block that keeps no state yet takes a tile at a time, to scan the rest once it does
-            int nk = evaluate ? 0 : scan || !g.tile_scan ? end - tile : 1;
+            int nk = evaluate ? 0 : scan || !g.tile_scan ? end - tile : min(1, end - tile);
             int k = 0;
             if (scan) {
                 if (axis == 0) scan_rows(g, tile, nk, v0, v1);
@@ -268,14 +271,14 @@ struct TilePass {
                     if (axis != 0) ds = g.tile_lines;
                     centre = (p.width / 2) * ds;      // the middle of the tile's first line
                     k++;
-                } else if (nk == 0 || !pack(all && tile + nk >= end, p, centre)) {
+                } else if (waiting || !pack(all && tile + nk >= end, p, centre)) {
                     break;
                 }
                 seen = compute(g, p, ds, centre);
                 evaluate = false;
             }
             tile += nk;
-        }
+        } while (tile < end);
         return next;
     }
 
@@ -840,6 +843,7 @@ __device__ __forceinline__ bool tile_arrive(TileCtl* ctl)
     if (threadIdx.x == 0) {
         __threadfence();
         is_last = atomicAdd(&ctl->arrived, 1u) == gridDim.x - 1;
+        __threadfence();
         if (is_last) {
             ctl->ticket = 0;
             ctl->arrived = 0;
@@ -892,6 +896,83 @@ tile_kernel(const __grid_constant__ SweepArgs<T> A, TileCtl* ctl, int last)
     if (tile_arrive(ctl) && threadIdx.x == 0) {
         if (ran) tile_clear_hints(A, P.src);
         if (last) tile_commit(A.state, A.cfg);
+    }
+}
+
+// Many independent domains in one launch (batch.cu).  Blocks [first[d], first[d + 1]) start on domain d,
+// in proportion to its cells, so that a block keeps the states of one domain; a domain's units beyond
+// its blocks' first ones come from its own ticket counter.  A block that finds its domain's units
+// taken joins the domain with the most units left.  The last block to finish commits every domain.
+template <class T, int SCHEME, int PROJ>
+__global__ void __launch_bounds__(kTileThreads, tile_min_blocks<T>())
+tile_batch_kernel(const SweepArgs<T>* __restrict__ doms, const int* __restrict__ first, const int* __restrict__ units,
+                  uint32_t* __restrict__ tickets, int ndom, int pass, TileCtl* ctl, int last)
+{
+    __shared__ TileShared<T> sh;
+    __shared__ __align__(16) SweepArgs<T> sA;
+    __shared__ unsigned long long pick;
+    const int tid = threadIdx.x;
+    TilePass<T, SCHEME, PROJ> P(sA, sh);
+    sh.acc[tid].init();
+    int d = batch_domain_index(first, ndom, blockIdx.x);
+    int u = (int)blockIdx.x - first[d];
+    for (;;) {
+        // the domain's arguments in shared memory: read once, and not aliased by the stores
+        __syncthreads();
+        {
+            static_assert(sizeof(SweepArgs<T>) % 4 == 0, "word copy");
+            const int* s = reinterpret_cast<const int*>(&doms[d]);
+            int* t = reinterpret_cast<int*>(&sA);
+            for (int w = tid; w < (int)(sizeof(SweepArgs<T>) / 4); w += kTileThreads) t[w] = s[w];
+        }
+        tile_forget(sh);
+        __syncthreads();
+        const int total = units[d];
+        const int given = first[d + 1] - first[d];
+        uint32_t* ticket = &tickets[d];
+        if (u < total) {
+            if (P.start(pass, last != 0, tid == 0)) {
+                while (u < total)
+                    u = P.unit(u, total, [&]() { return (int)(given + atomicAdd(ticket, 1u)); });
+                if (last) tile_flush(sh, sA.state);
+            } else if (tid == 0) {
+                atomicMax(ticket, (uint32_t)total);      // nothing to do here: no block joins it
+            }
+        }
+        // the domain with the most units left
+        __syncthreads();
+        if (tid == 0) pick = 0;
+        __syncthreads();
+        unsigned long long best = 0;
+        for (int k = tid; k < ndom; k += kTileThreads) {
+            const int left = units[k] - (first[k + 1] - first[k]) - (int)min(__ldcg(&tickets[k]), 0x3fffffffu);
+            if (left > 0) best = max(best, (unsigned long long)left << 32 | (unsigned)k);
+        }
+        if (best != 0) atomicMax(&pick, best);
+        __syncthreads();
+        if (pick == 0) break;
+        d = (int)(uint32_t)pick;
+        __syncthreads();
+        if (tid == 0) pick = atomicAdd(&tickets[d], 1u);
+        __syncthreads();
+        u = first[d + 1] - first[d] + (int)(uint32_t)pick;
+    }
+    if (tile_arrive(ctl)) {
+        for (int k = tid; k < ndom; k += kTileThreads) {
+            const SweepArgs<T>& A = doms[k];
+            tickets[k] = 0;
+            StepState st;
+            st.time = __ldcg(&A.state->time);
+            st.next_dt = __ldcg(&A.state->next_dt);
+            st.raw_dt = __ldcg(&A.state->raw_dt);
+            st.cycle = __ldcg(&A.state->cycle);
+            st.status = __ldcg(&A.state->status);
+            st.buf_base = __ldcg(&A.state->buf_base);
+            const CycleDt cd = cycle_time_step(st, A.cfg);
+            if (!cd.run || cd.invalid) continue;
+            tile_clear_hints(A, (int)(((int64_t)st.cycle * A.npass + pass + st.buf_base) & 1));
+            if (last) tile_commit(A.state, A.cfg);
+        }
     }
 }
 
