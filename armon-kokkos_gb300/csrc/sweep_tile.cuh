@@ -312,7 +312,9 @@ struct TilePass {
                 const int q = 32 * (i0 + i) + lane, t = a0 - H + q;
                 const bool out = q >= width, real = t >= 0 && t < g.n;
                 const uint32_t b0 = __ballot_sync(0xffffffffu, out || (real ? v0 && same_as_kept(c[i], 0) : v0 > 1));
-                const uint32_t b1 = __ballot_sync(0xffffffffu, out || (real ? v1 && same_as_kept(c[i], 1) : v1 > 1));
+                uint32_t b1 = 0;
+                if (v1 && b0 != 0xffffffffu)
+                    b1 = __ballot_sync(0xffffffffu, out || (real ? same_as_kept(c[i], 1) : v1 > 1));
                 if (lane == 0) {
                     sh.match[parity][0][w][i0 + i] = b0;
                     sh.match[parity][1][w][i0 + i] = b1;
@@ -350,6 +352,20 @@ struct TilePass {
         const uint32_t idle0 = __ballot_sync(0xffffffffu, e == 0), idle1 = __ballot_sync(0xffffffffu, e == 1);
         push(live & ~(idle0 | idle1), grp, a0, len);
         const int64_t base = A.origin + (int64_t)grp * g.lstride + a0;
+        const int whole = live == (idle0 & live) ? 0 : live == (idle1 & live) ? 1 : -1;
+        if (whole >= 0 && !pcg && a0 >= H && a0 + len <= g.n - H) {
+            // the whole tile, away from the walls
+            const T* kv = sh.kept[whole];
+            const T o0 = kv[kRunOut], o1 = kv[kRunOut + 1], o2 = kv[kRunOut + 2], o3 = kv[kRunOut + 3];
+            T* const* out = A.buf[src ^ 1];
+            T *rho = out[0] + base + lane, *ua = out[1 + axis] + base + lane, *uo = out[2 - axis] + base + lane, *E = out[3] + base + lane;
+#pragma unroll
+            for (int i = 0; i < kTileWarps; i++) {
+                if (32 * i + lane < len) { rho[32 * i] = o0; ua[32 * i] = o1; uo[32 * i] = o2; E[32 * i] = o3; }
+            }
+            count_kept(whole);
+            return;
+        }
         for (int o = lane; o < len; o += 32) {
             const int j = o >> 3;
             if ((idle0 >> j) & 1u) store_kept(g, base + o, a0 + o, 0);
@@ -387,9 +403,18 @@ struct TilePass {
             A.cmat[i] = kv[kRunC];
             A.gmat[i] = (1 + A.gamma) / 2;
         }
-        if (last && (wall || !((counted >> e) & 1u))) {
-            if (!wall) counted |= 1u << e;
-            add_dt(o, kv[kRunC]);
+        if (wall) {
+            if (last) add_dt(o, kv[kRunC]);
+        } else {
+            count_kept(e);
+        }
+    }
+    // A run of kept state e has been stored: its speeds count once.
+    __device__ __forceinline__ void count_kept(int e)
+    {
+        if (last && !((counted >> e) & 1u)) {
+            counted |= 1u << e;
+            add_dt(sh.kept[e] + kRunOut, sh.kept[e][kRunC]);
         }
     }
     // dt_CFL of the state after this pass, with c from this pass's EOS
@@ -475,8 +500,21 @@ struct TilePass {
         if (w < kTileWarps - 1) {
             // warp w stores chunk w of the uniform columns
             const int e = !col ? -1 : ((M0[w] & M0[w + 1]) >> lane) & 1u ? 0 : ((M1[w] & M1[w + 1]) >> lane) & 1u ? 1 : -1;
-            if (e >= 0) {
-                const int end = min(8 * w + 8, len);
+            const int end = min(8 * w + 8, len);
+            if (e >= 0 && !pcg && a0 >= H && a0 + len <= g.n - H) {
+                // away from the walls
+                const T* kv = sh.kept[e];
+                const T o0 = kv[kRunOut], o1 = kv[kRunOut + 1], o2 = kv[kRunOut + 2], o3 = kv[kRunOut + 3];
+                T* const* out = A.buf[src ^ 1];
+                const int64_t i0 = A.origin + (int64_t)line * g.lstride + (int64_t)(a0 + 8 * w) * g.s;
+                T *rho = out[0] + i0, *ua = out[1 + axis] + i0, *uo = out[2 - axis] + i0, *E = out[3] + i0;
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    if (8 * w + i < end) { *rho = o0; *ua = o1; *uo = o2; *E = o3; }
+                    rho += g.s; ua += g.s; uo += g.s; E += g.s;
+                }
+                if (8 * w < end) count_kept(e);
+            } else if (e >= 0) {
                 for (int o = 8 * w; o < end; o++) store_kept(g, A.origin + (int64_t)line * g.lstride + (int64_t)(a0 + o) * g.s, a0 + o, e);
             }
         } else if (col) {
