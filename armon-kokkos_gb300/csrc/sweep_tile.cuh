@@ -214,6 +214,13 @@ struct TilePass {
                same_bits(c.E, k[kRunE]);
     }
 
+    // Whether a loaded cell equals a kept state, read from shared memory each time (a state held in
+    // registers over a scan's loop costs 8 or 16 of them, and the loop's loads in flight spill).
+    static __device__ __forceinline__ bool same_cell(const T (&c)[4], const T* k)
+    {
+        return same_bits(c[0], k[kRunRho]) & same_bits(c[1], k[kRunUa]) & same_bits(c[2], k[kRunUo]) & same_bits(c[3], k[kRunE]);
+    }
+
     // The unit's tiles.  `after`, run by thread 0, gives the block's next unit, which is returned;
     // when there is none (>= total), what the list still holds is computed too.
     template <class After>
@@ -296,30 +303,36 @@ struct TilePass {
         if (grp >= g.nlines) return;
         const int a0 = seg * g.tile_len;
         const int width = min(g.n, a0 + g.tile_len) - a0 + 2 * H;
-        const int64_t base = A.origin + (int64_t)grp * g.lstride;
-        constexpr int kBatch = sizeof(T) == 8 ? 4 : 8;
+        // positions [lo, lo + real) of the tile are cells; the ones past its end match, ghosts as the state allows
+        const int lo = max(0, H - a0), real = min(width, g.n - a0 + H) - lo;
+        T* const* in = A.buf[src];
+        const int64_t i0 = A.origin + (int64_t)grp * g.lstride + (a0 - H) + lane;
+        const T *rho = in[0] + i0, *ua = in[1 + axis] + i0, *uo = in[2 - axis] + i0, *E = in[3] + i0;
+        const T *k0 = sh.kept[0], *k1 = sh.kept[1];
+        constexpr int kBatch = 4;
 #pragma unroll 1
         for (int i0 = 0; i0 < kTileWarps; i0 += kBatch) {
-            CellIn<T> c[kBatch];
+            T c[kBatch][4] = {};
 #pragma unroll
             for (int i = 0; i < kBatch; i++) {
-                c[i] = CellIn<T>{};
-                const int q = 32 * (i0 + i) + lane, t = a0 - H + q;
-                if (q < width && t >= 0 && t < g.n) load(base + t, c[i]);
+                if ((unsigned)(32 * (i0 + i) + lane - lo) < (unsigned)real) {
+                    c[i][0] = rho[32 * i]; c[i][1] = ua[32 * i]; c[i][2] = uo[32 * i]; c[i][3] = E[32 * i];
+                }
             }
 #pragma unroll
             for (int i = 0; i < kBatch; i++) {
-                const int q = 32 * (i0 + i) + lane, t = a0 - H + q;
-                const bool out = q >= width, real = t >= 0 && t < g.n;
-                const uint32_t b0 = __ballot_sync(0xffffffffu, out || (real ? v0 && same_as_kept(c[i], 0) : v0 > 1));
+                const int q = 32 * (i0 + i) + lane;
+                const bool cell = (unsigned)(q - lo) < (unsigned)real;
+                const uint32_t b0 = __ballot_sync(0xffffffffu, (cell & same_cell(c[i], k0) & (v0 != 0)) | (!cell & ((q >= width) | (v0 > 1))));
                 uint32_t b1 = 0;
                 if (v1 && b0 != 0xffffffffu)
-                    b1 = __ballot_sync(0xffffffffu, out || (real ? same_as_kept(c[i], 1) : v1 > 1));
+                    b1 = __ballot_sync(0xffffffffu, (cell & same_cell(c[i], k1)) | (!cell & ((q >= width) | (v1 > 1))));
                 if (lane == 0) {
                     sh.match[parity][0][w][i0 + i] = b0;
                     sh.match[parity][1][w][i0 + i] = b1;
                 }
             }
+            rho += 32 * kBatch; ua += 32 * kBatch; uo += 32 * kBatch; E += 32 * kBatch;
         }
         __syncwarp();
         if (__any_sync(0xffffffffu, chunk_state(w, lane) >= 0 && 8 * lane < width - 2 * H) && lane == 0)
@@ -451,25 +464,28 @@ struct TilePass {
         const bool col = lane < nk * g.tile_lines && line < g.nlines;
         const int a0 = seg * g.tile_len;
         const int width = min(g.n, a0 + g.tile_len) - a0 + 2 * H;
-        const int64_t base = A.origin + (int64_t)line * g.lstride;
-        constexpr int kBatch = sizeof(T) == 8 ? 4 : 8;
+        // positions [lo, lo + real) of the segment are cells
+        const int lo = max(0, H - a0), real = min(width, g.n - a0 + H) - lo;
+        T* const* in = A.buf[src];
+        const int64_t i0 = A.origin + (int64_t)line * g.lstride + (int64_t)(a0 - H + 8 * w) * g.s;
+        const T *rho = in[0] + i0, *ua = in[1 + axis] + i0, *uo = in[2 - axis] + i0, *E = in[3] + i0;
+        const T *k0 = sh.kept[0], *k1 = sh.kept[1];
+        constexpr int kBatch = 4;
         bool m0 = v0 != 0, m1 = v1 != 0;
         if (col) {
 #pragma unroll 1
-            for (int i0 = 0; i0 < 8; i0 += kBatch) {
-                CellIn<T> c[kBatch];
+            for (int q0 = 8 * w; q0 < 8 * w + 8; q0 += kBatch) {
+                T c[kBatch][4] = {};
 #pragma unroll
                 for (int i = 0; i < kBatch; i++) {
-                    c[i] = CellIn<T>{};
-                    const int q = 8 * w + i0 + i, t = a0 - H + q;
-                    if (q < width && t >= 0 && t < g.n) load(base + (int64_t)t * g.s, c[i]);
+                    if ((unsigned)(q0 + i - lo) < (unsigned)real) { c[i][0] = *rho; c[i][1] = *ua; c[i][2] = *uo; c[i][3] = *E; }
+                    rho += g.s; ua += g.s; uo += g.s; E += g.s;
                 }
 #pragma unroll
                 for (int i = 0; i < kBatch; i++) {
-                    const int q = 8 * w + i0 + i, t = a0 - H + q;
-                    const bool out = q >= width, real = t >= 0 && t < g.n;
-                    m0 = m0 && (out || (real ? same_as_kept(c[i], 0) : v0 > 1));
-                    m1 = m1 && (out || (real ? same_as_kept(c[i], 1) : v1 > 1));
+                    const bool cell = (unsigned)(q0 + i - lo) < (unsigned)real, out = q0 + i >= width;
+                    m0 = m0 & ((cell & same_cell(c[i], k0)) | (!cell & (out | (v0 > 1))));
+                    m1 = m1 & ((cell & same_cell(c[i], k1)) | (!cell & (out | (v1 > 1))));
                 }
             }
         }
