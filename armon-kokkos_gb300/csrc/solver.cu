@@ -126,7 +126,7 @@ void fill_geom(armon_solver* s, SweepArgs<T>& a)
         int units = 1;
         for (int axis = 0; axis < 2; axis++) {
             set_tile_axis(a.geom[axis], axis == 0, stencil_reach(&s->p), s->sm_count, slots,
-                          s->tile_lines > 0 ? s->tile_lines : kTileYLines);
+                          s->tile_lines > 0 ? s->tile_lines : tile_y_lines<T>());
             units = std::max(units, a.geom[axis].tile_units);
         }
         s->grid = std::min(slots, units);
@@ -396,7 +396,9 @@ int start_tuning(armon_solver* s)
     std::vector<int> forms;
     auto& T = s->tune;
     if (s->tile) {
-        for (int lines : {4, 8, 2}) T.cand.push_back(Tiling{0, lines, block, kTileForm});
+        // columns of a Y tile: the usual number and four
+        for (int lines : {s->fp32 ? tile_y_lines<float>() : tile_y_lines<double>(), 4})
+            T.cand.push_back(Tiling{0, lines, block, kTileForm});
     } else if (s->d_faces && s->o.split_pass == 0) forms = {1, 0}; else forms = {s->split ? 1 : 0};
     for (int form : forms) {
         const int per_sm = form ? sweep_split_blocks_per_sm(s->fp32, p.scheme, p.projection, block)

@@ -73,13 +73,18 @@ inline AxisTiling choose_segments(int n, int nlines, int block, int halo, int sm
     return axis_tiling(n, nlines, block, best_seg);
 }
 
-// Threads of a tile (sweep_tile.cuh), and the columns of a Y tile: four (FP64) are a sector.
+// Threads of a tile (sweep_tile.cuh), and the columns of a Y tile.  More columns read longer stretches
+// of a row, fewer leave longer tiles and less halo: two of 120 positions (halo 6 %), three of 72 or
+// four of 56 (13 %).  FP64, bound by its arithmetic, takes two (a 2048x2048 moving flow, 24 cycles:
+// 45.9 ms, against 47.5 with three or four); FP32 three (48 small domains: 17.5 ms, against 18.8 with
+// two and 18.5 with four; large domains within 1 %).
 constexpr int kTileBlock = 256;
-constexpr int kTileYLines = 4;
+template <class T> constexpr int tile_y_lines() { return sizeof(T) == 8 ? 2 : 3; }
 
 // The tiles of one axis.  A tile is `lines` lines by width = len + 2 halo positions, at most kTileBlock
 // threads.  Along rows (X) the positions are consecutive in memory, so a tile is as long as the block
-// allows; along columns (Y) the lines are, so a tile takes y_lines of them and what length is left.
+// allows; along columns (Y) the lines are, so a tile takes y_lines of them and what length is left, in
+// whole eights (a scan's threads take eight positions each).
 // The segments of a line are made equal.  A domain with fewer tiles than SMs takes fewer lines per
 // tile: a pass over it lasts as long as one position's chain, whatever a tile holds.  Large units
 // leave about four tiles per resident block to single-tile units, which end the launch evenly.
@@ -87,7 +92,7 @@ template <class T>
 void set_tile_axis(AxisGeom<T>& g, bool rows, int halo, int sms, int slots, int y_lines)
 {
     const int want = rows ? 1 : std::max(1, std::min(y_lines, g.nlines));
-    const int longest = std::max(1, std::min(248, kTileBlock / want - 2 * halo));
+    const int longest = std::max(1, rows ? std::min(248, kTileBlock - 2 * halo) : kTileBlock / want / 8 * 8 - 2 * halo);
     int segs = (g.n + longest - 1) / longest;
     const int len = (g.n + segs - 1) / segs;
     segs = (g.n + len - 1) / len;
@@ -99,7 +104,7 @@ void set_tile_axis(AxisGeom<T>& g, bool rows, int halo, int sms, int slots, int 
     g.tile_lines = std::max(1, std::min({rows ? fit : std::min(fit, want), g.nlines, spread}));
     g.tile_groups = (g.nlines + g.tile_lines - 1) / g.tile_lines;
     // worth a scan when a block has several tiles; the walls' positions may not overlap
-    g.tile_scan = (rows ? g.tile_lines == 1 : g.tile_lines * kTileUnit <= 32 && len <= 56) && g.n >= 32 &&
+    g.tile_scan = (rows ? g.tile_lines == 1 : g.tile_lines * kTileUnit <= 32 && (g.tile_width + 7) / 8 * 8 * g.tile_lines <= kTileBlock) && g.n >= 32 &&
                   (int64_t)segs * g.tile_groups >= 3 * (int64_t)slots;
     if (!rows && g.tile_scan)       // a large unit of columns lies in one segment
         g.tile_groups = (g.tile_groups + kTileUnit - 1) / kTileUnit * kTileUnit;

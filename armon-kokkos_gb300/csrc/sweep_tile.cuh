@@ -396,9 +396,12 @@ struct TilePass {
     __device__ __forceinline__ void push_run(uint32_t mask, int j, int line, int a0, int len)
     {
         const int chunks = __ffs((int)~mask) - 1;            // ones at the low end (mask has at most 31)
-        const int cells = min(8 * chunks, len - 8 * j);
+        list(line, a0 + 8 * j, min(8 * chunks, len - 8 * j));
+    }
+    __device__ __forceinline__ void list(int line, int start, int cells)
+    {
         const uint32_t at = atomicAdd(&sh.tail[parity], 1u);
-        sh.list[at % kTileList] = Stretch{line, ((a0 + 8 * j) << 8) | cells};
+        sh.list[at % kTileList] = Stretch{line, (start << 8) | cells};
     }
     // The results of position t, at index i, of a run of kept state e.
     __device__ __forceinline__ void store_kept(const AxisGeom<T>& g, int64_t i, int t, int e)
@@ -452,30 +455,33 @@ struct TilePass {
         else { p.q = r - kPlain - kSide; p.width = kSide; p.t = g.n - 2 * H + p.q; }
         return p;
     }
-    // Columns: the unit's tiles are columns line0 .. of one segment, a lane each; warp w takes positions
-    // 8 w .. 8 w + 7 of the segment (halo included), and match[state][0][w] has bit c set when they all
-    // match in column c.  Chunk j of a column is uniform when words j and j + 1 have its bit.
+    // Columns: the unit's nk tiles are `cols` columns of one segment; thread f takes column f % cols and
+    // the eight positions 8 (f / cols) .. of the segment (halo included), and bit f of match[state][0]
+    // says whether they all match.  Chunk j of a column is uniform when bits j cols + column and
+    // (j + 1) cols + column are set.
     __device__ __forceinline__ void scan_columns(const AxisGeom<T>& g, int tile0, int nk, int v0, int v1)
     {
-        const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
         int seg, grp;
         place(g, tile0, seg, grp);
-        const int line = grp * g.tile_lines + lane;
-        const bool col = lane < nk * g.tile_lines && line < g.nlines;
+        const int cols = nk * g.tile_lines;
+        const int j = tid / cols;
+        const int line = grp * g.tile_lines + tid - j * cols;
         const int a0 = seg * g.tile_len;
         const int width = min(g.n, a0 + g.tile_len) - a0 + 2 * H;
         // positions [lo, lo + real) of the segment are cells
         const int lo = max(0, H - a0), real = min(width, g.n - a0 + H) - lo;
         T* const* in = A.buf[src];
-        const int64_t i0 = A.origin + (int64_t)line * g.lstride + (int64_t)(a0 - H + 8 * w) * g.s;
+        const int64_t i0 = A.origin + (int64_t)line * g.lstride + (int64_t)(a0 - H + 8 * j) * g.s;
         const T *rho = in[0] + i0, *ua = in[1 + axis] + i0, *uo = in[2 - axis] + i0, *E = in[3] + i0;
         const T *k0 = sh.kept[0], *k1 = sh.kept[1];
         constexpr int kBatch = 4;
         bool m0 = v0 != 0, m1 = v1 != 0;
-        if (col) {
+        const bool live = line < g.nlines && 8 * j < width;
+        if (live) {
 #pragma unroll 1
-            for (int q0 = 8 * w; q0 < 8 * w + 8; q0 += kBatch) {
-                T c[kBatch][4] = {};
+            for (int q0 = 8 * j; q0 < 8 * j + 8; q0 += kBatch) {
+                T c[kBatch][4] = {};      // (left unset, they would be carried from batch to batch)
 #pragma unroll
                 for (int i = 0; i < kBatch; i++) {
                     if ((unsigned)(q0 + i - lo) < (unsigned)real) { c[i][0] = *rho; c[i][1] = *ua; c[i][2] = *uo; c[i][3] = *E; }
@@ -495,52 +501,62 @@ struct TilePass {
             sh.match[parity][1][0][w] = b1;
         }
         __syncthreads();
-        if (w < kTileWarps - 1) {
-            const uint32_t idle = (sh.match[parity][0][0][w] & sh.match[parity][0][0][w + 1]) |
-                                  (sh.match[parity][1][0][w] & sh.match[parity][1][0][w + 1]);
-            if (__any_sync(0xffffffffu, col && ((idle >> lane) & 1u) && 8 * w < width - 2 * H) && lane == 0)
-                sh.uniform[parity] = 1;
+        if (__any_sync(0xffffffffu, live && 8 * j < width - 2 * H && column_state(tid, cols) >= 0) && lane == 0)
+            sh.uniform[parity] = 1;
+    }
+    // The kept state of the chunk that begins with thread f's positions, -1 when its windows do not all
+    // hold one.  (A segment's last chunk may lack positions past its halo: they would match.)
+    __device__ __forceinline__ int column_state(int f, int cols) const
+    {
+        const int h = f + cols;
+        const bool past = h >= kTileThreads;
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            const uint32_t* m = &sh.match[parity][e][0][0];
+            if (((m[f >> 5] >> (f & 31)) & 1u) && (past || ((m[(h & 255) >> 5] >> (h & 31)) & 1u))) return e;
         }
+        return -1;
     }
     __device__ __forceinline__ void fill_columns(const AxisGeom<T>& g, int tile0, int nk)
     {
-        const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        const int tid = threadIdx.x;
         int seg, grp;
         place(g, tile0, seg, grp);
-        const int line = grp * g.tile_lines + lane;
-        const bool col = lane < nk * g.tile_lines && line < g.nlines;
+        const int cols = nk * g.tile_lines;
+        const int j = tid / cols;
+        const int line = grp * g.tile_lines + tid - j * cols;
+        if (line >= g.nlines) return;
         const int a0 = seg * g.tile_len;
         const int len = min(g.n, a0 + g.tile_len) - a0;
-        const uint32_t* M0 = &sh.match[parity][0][0][0];
-        const uint32_t* M1 = &sh.match[parity][1][0][0];
-        if (w < kTileWarps - 1) {
-            // warp w stores chunk w of the uniform columns
-            const int e = !col ? -1 : ((M0[w] & M0[w + 1]) >> lane) & 1u ? 0 : ((M1[w] & M1[w + 1]) >> lane) & 1u ? 1 : -1;
-            const int end = min(8 * w + 8, len);
-            if (e >= 0 && !pcg && a0 >= H && a0 + len <= g.n - H) {
-                // away from the walls
-                const T* kv = sh.kept[e];
-                const T o0 = kv[kRunOut], o1 = kv[kRunOut + 1], o2 = kv[kRunOut + 2], o3 = kv[kRunOut + 3];
-                T* const* out = A.buf[src ^ 1];
-                const int64_t i0 = A.origin + (int64_t)line * g.lstride + (int64_t)(a0 + 8 * w) * g.s;
-                T *rho = out[0] + i0, *ua = out[1 + axis] + i0, *uo = out[2 - axis] + i0, *E = out[3] + i0;
+        const int end = min(8 * j + 8, len);
+        const int e = 8 * j < len ? column_state(tid, cols) : -1;
+        if (e >= 0 && !pcg && a0 >= H && a0 + len <= g.n - H) {
+            // away from the walls
+            const T* kv = sh.kept[e];
+            const T o0 = kv[kRunOut], o1 = kv[kRunOut + 1], o2 = kv[kRunOut + 2], o3 = kv[kRunOut + 3];
+            T* const* out = A.buf[src ^ 1];
+            const int64_t i0 = A.origin + (int64_t)line * g.lstride + (int64_t)(a0 + 8 * j) * g.s;
+            T *rho = out[0] + i0, *ua = out[1 + axis] + i0, *uo = out[2 - axis] + i0, *E = out[3] + i0;
 #pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    if (8 * w + i < end) { *rho = o0; *ua = o1; *uo = o2; *E = o3; }
-                    rho += g.s; ua += g.s; uo += g.s; E += g.s;
-                }
-                if (8 * w < end) count_kept(e);
-            } else if (e >= 0) {
-                for (int o = 8 * w; o < end; o++) store_kept(g, A.origin + (int64_t)line * g.lstride + (int64_t)(a0 + o) * g.s, a0 + o, e);
+            for (int i = 0; i < 8; i++) {
+                if (8 * j + i < end) { *rho = o0; *ua = o1; *uo = o2; *E = o3; }
+                rho += g.s; ua += g.s; uo += g.s; E += g.s;
             }
-        } else if (col) {
-            // the last warp lists the others' chunks, a lane per column
-            uint32_t todo = 0;
-            for (int j = 0; 8 * j < len; j++)
-                if (!((((M0[j] & M0[j + 1]) | (M1[j] & M1[j + 1])) >> lane) & 1u)) todo |= 1u << j;
-            todo |= (todo << 1) & (todo >> 1);
-            for (int j = 0; todo >> j; j++)
-                if (((todo >> j) & 1u) && (j == 0 || !((todo >> (j - 1)) & 1u))) push_run(todo >> j, j, line, a0, len);
+            count_kept(e);
+        } else if (e >= 0) {
+            for (int o = 8 * j; o < end; o++)
+                store_kept(g, A.origin + (int64_t)line * g.lstride + (int64_t)(a0 + o) * g.s, a0 + o, e);
+        }
+        // a run's first thread lists it; runs one chunk apart are joined, as push does
+        const auto todo = [&](int k) { return k >= 0 && 8 * k < len && column_state(tid + (k - j) * cols, cols) < 0; };
+        if (8 * j < len && e < 0 && !todo(j - 1) && !todo(j - 2)) {
+            int k = j + 1;
+            for (;;) {
+                if (todo(k)) k++;
+                else if (todo(k + 1)) k += 2;
+                else break;
+            }
+            list(line, a0 + 8 * j, min(8 * k, len) - 8 * j);
         }
     }
 
