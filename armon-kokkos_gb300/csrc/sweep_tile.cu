@@ -10,7 +10,10 @@ namespace {
 template <class T, int S, int P>
 cudaError_t launch_tile_one(const SweepArgs<T>& a, TileCtl* ctl, bool last, int grid, cudaStream_t st)
 {
-    tile_kernel<T, S, P><<<grid, kTileThreads, 0, st>>>(a, ctl, last ? 1 : 0);
+    if (a.reuse && (a.geom[0].tile_scan || a.geom[1].tile_scan))
+        tile_kernel<T, S, P, true><<<grid, kTileThreads, 0, st>>>(a, ctl, last ? 1 : 0);
+    else
+        tile_kernel<T, S, P, false><<<grid, kTileThreads, 0, st>>>(a, ctl, last ? 1 : 0);
     return cudaGetLastError();
 }
 
@@ -28,11 +31,11 @@ int tile_blocks_t(int scheme, int proj)
     int n = 0;
     cudaError_t e;
     if (scheme == 1)
-        e = proj == 2 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, tile_kernel<T, 1, 2>, kTileThreads, 0)
-                      : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, tile_kernel<T, 1, 1>, kTileThreads, 0);
+        e = proj == 2 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, tile_kernel<T, 1, 2, true>, kTileThreads, 0)
+                      : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, tile_kernel<T, 1, 1, true>, kTileThreads, 0);
     else
-        e = proj == 2 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, tile_kernel<T, 0, 2>, kTileThreads, 0)
-                      : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, tile_kernel<T, 0, 1>, kTileThreads, 0);
+        e = proj == 2 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, tile_kernel<T, 0, 2, true>, kTileThreads, 0)
+                      : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, tile_kernel<T, 0, 1, true>, kTileThreads, 0);
     return (e == cudaSuccess && n > 0) ? n : 1;
 }
 

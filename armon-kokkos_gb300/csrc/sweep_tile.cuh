@@ -89,8 +89,9 @@ struct TileShared {
     int next[2];                      // [unit parity]: the block's next unit
 };
 
-// The tiles of one unit of one domain.
-template <class T, int SCHEME, int PROJ>
+// The tiles of one unit of one domain.  SCAN: its units may be scanned (AxisGeom::tile_scan); without it
+// the pass is its stages alone, half the code.
+template <class T, int SCHEME, int PROJ, bool SCAN>
 struct TilePass {
     static constexpr bool kGAD = SCHEME == 1;
     static constexpr bool kE2 = PROJ == 2;
@@ -142,7 +143,7 @@ struct TilePass {
             tile_q = tid / g.tile_lines;
             tile_l = tid - tile_q * g.tile_lines;
         }
-        hints = A.reuse && g.tile_scan && A.sw >= H &&
+        hints = SCAN && A.reuse && g.tile_scan && A.sw >= H &&
                 (__ldcg(&A.hints->valid[src][0]) | __ldcg(&A.hints->valid[src][1])) != 0;
         return true;
     }
@@ -245,9 +246,9 @@ struct TilePass {
             const bool waiting = hints;      // only the hinted states this time
             bool evaluate = hints;
             hints = false;
-            const bool scan = g.tile_scan && (v0 | v1) && !evaluate && tile < end;
+            const bool scan = SCAN && g.tile_scan && (v0 | v1) && !evaluate && tile < end;
             // a block that keeps no state yet takes a tile at a time, to scan the rest once it does
-            int nk = evaluate ? 0 : scan || !g.tile_scan ? end - tile : min(1, end - tile);
+            int nk = evaluate ? 0 : scan || !SCAN || !g.tile_scan ? end - tile : min(1, end - tile);
             int k = 0;
             if (scan) {
                 if (axis == 0) scan_rows(g, tile, nk, v0, v1);
@@ -267,7 +268,7 @@ struct TilePass {
             for (;;) {
                 Spot p;
                 int ds = 1, centre = -1;
-                if (evaluate) {
+                if (SCAN && evaluate) {
                     p = hint_spot(g);
                 } else if (k < nk) {
                     if (scan && seen != claims) {   // a state more is kept: scan the rest again
@@ -278,7 +279,7 @@ struct TilePass {
                     if (axis != 0) ds = g.tile_lines;
                     centre = (p.width / 2) * ds;      // the middle of the tile's first line
                     k++;
-                } else if (waiting || !pack(all && tile + nk >= end, p, centre)) {
+                } else if (!SCAN || waiting || !pack(all && tile + nk >= end, p, centre)) {
                     break;
                 }
                 seen = compute(g, p, ds, centre);
@@ -659,7 +660,7 @@ struct TilePass {
             int m, side;
             const bool stale = source(g.n, p.t, m, side);
             const int64_t i = p.base + (int64_t)m * g.s;
-            if (p.hint >= 0) {
+            if (SCAN && p.hint >= 0) {
                 const T* v = A.hints->v[src][p.hint];
                 c.rho = __ldcg(v);
                 c.ua = __ldcg(v + 1 + axis);
@@ -690,7 +691,7 @@ struct TilePass {
             ARMON_X(13) = c.dm;
             sh.c[tid] = c.c;
         }
-        if (A.reuse && g.tile_scan) {
+        if (SCAN && A.reuse && g.tile_scan) {
             if (p.hint >= 0) {
                 if (on && q == H && width == 2 * H + 1) rec = p.hint;
             } else if ((tid >> 5) == (centre >> 5)) {
@@ -823,7 +824,7 @@ struct TilePass {
             o[1] = qdiv_at<8>(ra, inv_rho);
             o[2] = qdiv_at<8>(ro, inv_rho);
             o[3] = qdiv_at<8>(rE, inv_rho);
-            if (p.hint < 0) {
+            if (!SCAN || p.hint < 0) {
                 const int64_t i = p.base + (int64_t)p.t * g.s;
                 T* const* out = A.buf[src ^ 1];
                 out[0][i] = o[0];
@@ -943,12 +944,12 @@ __device__ __forceinline__ void tile_forget(TileShared<T>& sh)
 }
 
 // One domain.
-template <class T, int SCHEME, int PROJ>
+template <class T, int SCHEME, int PROJ, bool SCAN>
 __global__ void __launch_bounds__(kTileThreads, tile_min_blocks<T>())
 tile_kernel(const __grid_constant__ SweepArgs<T> A, TileCtl* ctl, int last)
 {
     __shared__ TileShared<T> sh;
-    TilePass<T, SCHEME, PROJ> P(A, sh);
+    TilePass<T, SCHEME, PROJ, SCAN> P(A, sh);
     tile_forget(sh);
     sh.acc[threadIdx.x].init();
     const bool ran = P.start(A.pass, last != 0, blockIdx.x == 0 && threadIdx.x == 0);
@@ -982,7 +983,7 @@ tile_batch_kernel(const SweepArgs<T>* __restrict__ doms, const int* __restrict__
     __shared__ __align__(16) SweepArgs<T> sA;
     __shared__ unsigned long long pick;
     const int tid = threadIdx.x;
-    TilePass<T, SCHEME, PROJ> P(sA, sh);
+    TilePass<T, SCHEME, PROJ, true> P(sA, sh);
     sh.acc[tid].init();
     int d = batch_domain_index(first, ndom, blockIdx.x);
     int u = (int)blockIdx.x - first[d];
