@@ -5,7 +5,13 @@
 // (k in [range.start, range.end), cell = inner_range.scale_index(k)) with one thread per index and
 // the reference's expression tree; the file is built with --fmad=false so every stage is bit-exact
 // with the reference's strict FP64 build.  These are the drop-in stages and the step-level checks;
-// the fused solver (sweep.cuh) is the fast path.
+// the solver (sweep_tile.cuh) is the fast path.
+//
+// What bounds a stage here is GB300's FP64 pipe (2 operations per SM per clock), where a division or
+// a square root takes ~10 slots, and 64-bit index divisions: the stages share the solver's exact
+// integer-pipe operations (softfp.cuh, the stage functions of sweep.cuh), and indexes below 2^32
+// divide in 32 bits.  A host program's 4 cycles at 1500x1000 (GAD, second order): 10.0 ms with the
+// hardware's divisions, 4.5 ms so.
 #include <cfloat>
 #include <cmath>
 #include <cstdio>
@@ -20,6 +26,7 @@
 #include "armon_kernels.h"
 #include "device_common.cuh"
 #include "init.cuh"
+#include "sweep.cuh"
 
 using armon::kmax;
 using armon::kmin;
@@ -36,8 +43,15 @@ cudaStream_t g_stream = nullptr;
 
 __host__ __device__ inline int64_t scale2d(const InnerRange2D& r, uint64_t i)
 {
-    int64_t ix = (int64_t)(i / r.row_range_length);
-    int64_t iy = (int64_t)(i % r.row_range_length);
+    int64_t ix, iy;
+    if (((i | (uint64_t)r.row_range_length) >> 32) == 0) {
+        const uint32_t n = (uint32_t)r.row_range_length, q = (uint32_t)i / n;
+        ix = q;
+        iy = (uint32_t)i - q * n;
+    } else {
+        ix = (int64_t)(i / r.row_range_length);
+        iy = (int64_t)(i % r.row_range_length);
+    }
     int64_t j = r.main_range_start + ix * r.main_range_step;
     return r.row_range_start + iy + j;
 }
@@ -124,31 +138,25 @@ double* scratch(size_t doubles)
     return buf[dev];
 }
 
-__device__ __forceinline__ void godunov(double rho_i, double rho_im, double c_i, double c_im, double u_i, double u_im,
-                                        double p_i, double p_im, double& us, double& ps)
+// A cell's values for a face flux (src/kernels/acoustic.cpp:10-19).
+__device__ __forceinline__ armon::CellIn<double> flux_cell(double rho, double c, double u, double p)
 {
-    // src/kernels/acoustic.cpp:10-19
-    double rc_l = rho_im * c_im;
-    double rc_r = rho_i * c_i;
-    us = (rc_l * u_im + rc_r * u_i + (p_im - p_i)) / (rc_l + rc_r);
-    ps = (rc_r * p_im + rc_l * p_i + rc_l * rc_r * (u_im - u_i)) / (rc_l + rc_r);
+    armon::CellIn<double> x{};
+    x.rho = rho;
+    x.ua = u;
+    x.p = p;
+    x.rc = rho * c;
+    x.rcu = x.rc * u;
+    return x;
 }
 
-__device__ __forceinline__ double limiter(int L, double r)
+// min over the two axes of the CFL length over the speed, of one index (src/kernels/reductions.cpp:16-20)
+__device__ __forceinline__ double dt_cell(double dx, double dy, double u, double v, double c, double mask)
 {
-    // src/kernels/limiters.h:15-34
-    if (L == 1) return kmax(0.0, kmin(1.0, r));
-    if (L == 2) return kmax(kmax(0.0, kmin(1.0, 2 * r)), kmin(2.0, r));
-    return 1.0;
-}
-
-__device__ __forceinline__ double slope_minmod(double u_im, double u_i, double u_ip, double r_m, double r_p)
-{
-    // src/kernels/euler_projection.cpp:73-79
-    double D_u_p = r_p * (u_ip - u_i);
-    double D_u_m = r_m * (u_i - u_im);
-    double s = copysign(1.0, D_u_p);
-    return s * kmax(0.0, kmin(s * D_u_p, s * D_u_m));
+    using armon::sfp::absval;
+    const double max_cx = armon::qmax(absval(u + c), absval(u - c)) * mask;
+    const double max_cy = armon::qmax(absval(v + c), absval(v - c)) * mask;
+    return armon::qmin(armon::sfp::div(dx, max_cx), armon::sfp::div(dy, max_cy));
 }
 
 __global__ void dt_partial_kernel(int64_t start, int64_t end, InnerRange1D ir, double dx, double dy, const double* umat,
@@ -159,9 +167,7 @@ __global__ void dt_partial_kernel(int64_t start, int64_t end, InnerRange1D ir, d
     double acc = DBL_MAX;
     for (int64_t k = start + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < end; k += (int64_t)gridDim.x * blockDim.x) {
         int64_t i = scale1d(ir, (uint64_t)k);
-        double max_cx = kmax(fabs(umat[i] + cmat[i]), fabs(umat[i] - cmat[i])) * mask[i];
-        double max_cy = kmax(fabs(vmat[i] + cmat[i]), fabs(vmat[i] - cmat[i])) * mask[i];
-        acc = kmin(acc, kmin(dx / max_cx, dy / max_cy));
+        acc = armon::qmin(acc, dt_cell(dx, dy, umat[i], vmat[i], cmat[i], mask[i]));
     }
     red[threadIdx.x] = acc;
     __syncthreads();
@@ -170,15 +176,6 @@ __global__ void dt_partial_kernel(int64_t start, int64_t end, InnerRange1D ir, d
         __syncthreads();
     }
     if (threadIdx.x == 0) partials[blockIdx.x] = red[0];
-}
-
-__global__ void min_final_kernel(const double* partials, int n, double* out)
-{
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        double acc = DBL_MAX;
-        for (int b = 0; b < n; b++) if (partials[b] < acc) acc = partials[b];
-        out[0] = acc;
-    }
 }
 
 __global__ void cons_partial_kernel(int64_t start, int64_t end, InnerRange1D ir, double ds, const double* rho,
@@ -234,9 +231,7 @@ __global__ void dt_tile_kernel(int64_t start, int64_t end, InnerRange1D ir, doub
     const int64_t t1 = min(end, t0 + kNoAllocTile);
     for (int64_t k = t0 + threadIdx.x; k < t1; k += blockDim.x) {
         int64_t i = scale1d(ir, (uint64_t)k);
-        double max_cx = kmax(fabs(umat[i] + cmat[i]), fabs(umat[i] - cmat[i])) * mask[i];
-        double max_cy = kmax(fabs(vmat[i] + cmat[i]), fabs(vmat[i] - cmat[i])) * mask[i];
-        acc = kmin(acc, kmin(dx / max_cx, dy / max_cy));
+        acc = armon::qmin(acc, dt_cell(dx, dy, umat[i], vmat[i], cmat[i], mask[i]));
     }
     red[threadIdx.x] = acc;
     __syncthreads();
@@ -302,10 +297,10 @@ void acoustic(const Range* range, const InnerRange2D* inner_range, Idx s, view* 
         const double *r = rho->data, *uu = u->data, *p = pmat->data, *c = cmat->data;
         launch_range(range, [=] __device__(int64_t k) {
             int64_t i = scale2d(ir, (uint64_t)k);
-            double a, b;
-            godunov(r[i], r[i - s], c[i], c[i - s], uu[i], uu[i - s], p[i], p[i - s], a, b);
-            us[i] = a;
-            ps[i] = b;
+            const armon::God<double> G = armon::godunov(flux_cell(r[i - s], c[i - s], uu[i - s], p[i - s]),
+                                                        flux_cell(r[i], c[i], uu[i], p[i]));
+            us[i] = G.us;
+            ps[i] = G.ps;
         });
     });
 }
@@ -324,27 +319,15 @@ void acoustic_GAD(const Range* range, const InnerRange2D* inner_range, Idx s, fl
         launch_range(range, [=] __device__(int64_t k) {
             // src/kernels/acoustic.cpp:40-88
             int64_t i = scale2d(ir, (uint64_t)k);
-            double ustar_im, pstar_im, ustar_i, pstar_i, ustar_ip, pstar_ip;
-            godunov(rh[i - s], rh[i - 2 * s], c[i - s], c[i - 2 * s], uu[i - s], uu[i - 2 * s], p[i - s], p[i - 2 * s],
-                    ustar_im, pstar_im);
-            godunov(rh[i], rh[i - s], c[i], c[i - s], uu[i], uu[i - s], p[i], p[i - s], ustar_i, pstar_i);
-            godunov(rh[i + s], rh[i], c[i + s], c[i], uu[i + s], uu[i], p[i + s], p[i], ustar_ip, pstar_ip);
-            double r_um = (ustar_ip - uu[i]) / (ustar_i - uu[i - s] + 1e-6);
-            double r_pm = (pstar_ip - p[i]) / (pstar_i - p[i - s] + 1e-6);
-            double r_up = (uu[i - s] - ustar_im) / (uu[i] - ustar_i + 1e-6);
-            double r_pp = (p[i - s] - pstar_im) / (p[i] - pstar_i + 1e-6);
-            r_um = limiter(L, r_um);
-            r_pm = limiter(L, r_pm);
-            r_up = limiter(L, r_up);
-            r_pp = limiter(L, r_pp);
-            double dm_l = rh[i - s] * dx;
-            double dm_r = rh[i] * dx;
-            double Dm = (dm_l + dm_r) / 2;
-            double rc_l = rh[i - s] * c[i - s];
-            double rc_r = rh[i] * c[i];
-            double theta = 0.5 * (1 - (rc_l + rc_r) / 2 * (dt / Dm));
-            ust[i] = ustar_i + theta * (r_up * (uu[i] - ustar_i) - r_um * (ustar_i - uu[i - s]));
-            pst[i] = pstar_i + theta * (r_pp * (p[i] - pstar_i) - r_pm * (pstar_i - p[i - s]));
+            const auto cell = [&](int64_t j) { return flux_cell(rh[j], c[j], uu[j], p[j]); };
+            const armon::CellIn<double> Cm = cell(i - 2 * s), Cl = cell(i - s), Cr = cell(i), Cp = cell(i + s);
+            const armon::God<double> G = armon::godunov(Cl, Cr);
+            const armon::GadDiff<double> Dm = armon::gad_diff(armon::godunov(Cm, Cl), Cm, Cl);
+            const armon::GadDiff<double> D = armon::gad_diff(G, Cl, Cr);
+            const armon::GadDiff<double> Dp = armon::gad_diff(armon::godunov(Cr, Cp), Cr, Cp);
+            const armon::Flux<double> f = armon::gad(G, Dm, D, Dp, Cl.rho * dx, Cr.rho * dx, L, dt);
+            ust[i] = f.us;
+            pst[i] = f.ps;
         });
     });
 }
@@ -358,13 +341,16 @@ void perfect_gas_EOS(const Range* range, const InnerRange2D* inner_range, flt_t 
         const InnerRange2D ir = *inner_range;
         const double *r = rho->data, *E = Emat->data, *u = umat->data, *v = vmat->data;
         double *p = pmat->data, *c = cmat->data, *g = gmat->data;
+        const double gamma_m1 = gamma - 1, half_sum = (1 + gamma) / 2;
         launch_range(range, [=] __device__(int64_t k) {
             // src/kernels/fluid_eos.cpp:17-21 (Kokkos::pow(x, 2) == x * x)
             int64_t i = scale2d(ir, (uint64_t)k);
-            double e = E[i] - 0.5 * (u[i] * u[i] + v[i] * v[i]);
-            p[i] = (gamma - 1) * r[i] * e;
-            c[i] = sqrt(gamma * p[i] / r[i]);
-            g[i] = (1 + gamma) / 2;
+            const double rho_i = r[i], u_i = u[i], v_i = v[i];
+            const double e = E[i] - armon::sfp::half(u_i * u_i + v_i * v_i);
+            const double p_i = gamma_m1 * rho_i * e;
+            p[i] = p_i;
+            c[i] = armon::sfp::sqrt(armon::sfp::div(gamma * p_i, rho_i));
+            g[i] = half_sum;
         });
     });
 }
@@ -416,10 +402,12 @@ void cell_update(const Range* range, const InnerRange2D* inner_range, Idx s, flt
         launch_range(range, [=] __device__(int64_t k) {
             // src/kernels/euler_projection.cpp:16-20
             int64_t i = scale2d(ir, (uint64_t)k);
-            double dm = r[i] * dx;
-            r[i] = dm / (dx + dt * (us[i + s] - us[i]));
-            uu[i] += dt / dm * (ps[i] - ps[i + s]);
-            E[i] += dt / dm * (ps[i] * us[i] - ps[i + s] * us[i + s]);
+            const double us0 = us[i], us1 = us[i + s], ps0 = ps[i], ps1 = ps[i + s];
+            const double dm = r[i] * dx;
+            const double dtdm = armon::sfp::div(dt, dm);
+            r[i] = armon::sfp::div(dm, dx + dt * (us1 - us0));
+            uu[i] += dtdm * (ps0 - ps1);
+            E[i] += dtdm * (ps0 * us0 - ps1 * us1);
         });
     });
 }
@@ -438,15 +426,18 @@ void euler_projection(const Range* range, const InnerRange2D* inner_range, Idx s
         launch_range(range, [=] __device__(int64_t k) {
             // src/kernels/euler_projection.cpp:34-46
             int64_t i = scale2d(ir, (uint64_t)k);
-            double dX = dx + dt * (us[i + s] - us[i]);
-            double tmp_rho = (dX * r[i] - (ar[i + s] - ar[i])) / dx;
-            double tmp_urho = (dX * r[i] * u[i] - (au[i + s] - au[i])) / dx;
-            double tmp_vrho = (dX * r[i] * v[i] - (av[i + s] - av[i])) / dx;
-            double tmp_Erho = (dX * r[i] * E[i] - (aE[i + s] - aE[i])) / dx;
+            const double dX = dx + dt * (us[i + s] - us[i]);
+            const double dXr = dX * r[i];
+            const armon::sfp::Recip per_dx = armon::sfp::recip(dx);
+            const double tmp_rho = armon::sfp::div(dXr - (ar[i + s] - ar[i]), per_dx, dx);
+            const double tmp_urho = armon::sfp::div(dXr * u[i] - (au[i + s] - au[i]), per_dx, dx);
+            const double tmp_vrho = armon::sfp::div(dXr * v[i] - (av[i + s] - av[i]), per_dx, dx);
+            const double tmp_Erho = armon::sfp::div(dXr * E[i] - (aE[i + s] - aE[i]), per_dx, dx);
+            const armon::sfp::Recip per_rho = armon::sfp::recip(tmp_rho);
             r[i] = tmp_rho;
-            u[i] = tmp_urho / tmp_rho;
-            v[i] = tmp_vrho / tmp_rho;
-            E[i] = tmp_Erho / tmp_rho;
+            u[i] = armon::sfp::div(tmp_urho, per_rho, tmp_rho);
+            v[i] = armon::sfp::div(tmp_vrho, per_rho, tmp_rho);
+            E[i] = armon::sfp::div(tmp_Erho, per_rho, tmp_rho);
         });
     });
 }
@@ -491,26 +482,28 @@ void advection_second_order(const Range* range, const InnerRange2D* inner_range,
             int64_t is = i;
             double disp = dt * us[i];
             double Dx;
-            if (disp > 0) {
+            if (armon::qgt0(disp)) {
                 Dx = -(dx - dt * us[i - s]);
                 i = i - s;
             } else {
                 Dx = dx + dt * us[i + s];
             }
-            double Dx_lm = dx + dt * (us[i] - us[i - s]);
-            double Dx_l = dx + dt * (us[i + s] - us[i]);
-            double Dx_lp = dx + dt * (us[i + 2 * s] - us[i + s]);
-            double r_m = (2 * Dx_l) / (Dx_l + Dx_lm);
-            double r_p = (2 * Dx_l) / (Dx_l + Dx_lp);
-            double slope_r = slope_minmod(r[i - s], r[i], r[i + s], r_m, r_p);
-            double slope_ur = slope_minmod(r[i - s] * u[i - s], r[i] * u[i], r[i + s] * u[i + s], r_m, r_p);
-            double slope_vr = slope_minmod(r[i - s] * v[i - s], r[i] * v[i], r[i + s] * v[i + s], r_m, r_p);
-            double slope_Er = slope_minmod(r[i - s] * E[i - s], r[i] * E[i], r[i + s] * E[i + s], r_m, r_p);
-            double length_factor = Dx / (2 * Dx_l);
-            ar[is] = disp * (r[i] - slope_r * length_factor);
-            au[is] = disp * (r[i] * u[i] - slope_ur * length_factor);
-            av[is] = disp * (r[i] * v[i] - slope_vr * length_factor);
-            aE[is] = disp * (r[i] * E[i] - slope_Er * length_factor);
+            const double us0 = us[i], us1 = us[i + s];
+            const double Dx_lm = dx + dt * (us0 - us[i - s]);
+            const double Dx_l = dx + dt * (us1 - us0);
+            const double Dx_lp = dx + dt * (us[i + 2 * s] - us1);
+            const auto cell = [&](int64_t j) {
+                const double rj = r[j];
+                return armon::Adv<double>{rj, rj * u[j], rj * v[j], rj * E[j]};
+            };
+            const armon::Adv<double> q0 = cell(i - s), q1 = cell(i), q2 = cell(i + s);
+            const armon::Adv<double> dm{q1.r - q0.r, q1.ra - q0.ra, q1.ro - q0.ro, q1.rE - q0.rE};
+            const armon::Adv<double> dp{q2.r - q1.r, q2.ra - q1.ra, q2.ro - q1.ro, q2.rE - q1.rE};
+            const armon::Adv<double> f = armon::advect2_upwind(disp, Dx, Dx_l, q1, dm, dp, Dx_l + Dx_lm, Dx_l + Dx_lp);
+            ar[is] = f.r;
+            au[is] = f.ra;
+            av[is] = f.ro;
+            aE[is] = f.rE;
         });
     });
 }
@@ -645,7 +638,7 @@ flt_t dt_CFL(const Range* range, const InnerRange1D* inner_range, flt_t dx, flt_
         if (n <= 0) { result = DBL_MAX; return; }
         dt_partial_kernel<<<kReduceBlocks, 256, 0, g_stream>>>(range->start, range->end, *inner_range, dx, dy, umat->data,
                                                                vmat->data, cmat->data, domain_mask->data, buf);
-        min_final_kernel<<<1, 32, 0, g_stream>>>(buf, kReduceBlocks, buf + kReduceBlocks);
+        min_tiles_kernel<<<1, 1024, 0, g_stream>>>(buf, kReduceBlocks, buf + kReduceBlocks);
         check_cuda(cudaGetLastError(), "dt_CFL launch");
         check_cuda(cudaMemcpyAsync(&result, buf + kReduceBlocks, sizeof(double), cudaMemcpyDeviceToHost, g_stream),
                    "dt_CFL copy");
