@@ -126,7 +126,7 @@ void fill_geom(armon_solver* s, SweepArgs<T>& a)
         int units = 1;
         for (int axis = 0; axis < 2; axis++) {
             set_tile_axis(a.geom[axis], axis == 0, stencil_reach(&s->p), s->sm_count, slots,
-                          s->tile_lines > 0 ? s->tile_lines : tile_y_lines<T>());
+                          s->tile_lines > 0 ? s->tile_lines : tile_y_lines<T>(), s->fp32 ? 4 : 8);
             units = std::max(units, a.geom[axis].tile_units);
         }
         s->grid = std::min(slots, units);

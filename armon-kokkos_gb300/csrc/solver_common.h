@@ -87,9 +87,12 @@ template <class T> constexpr int tile_y_lines() { return sizeof(T) == 8 ? 2 : 3;
 // whole eights (a scan's threads take eight positions each).
 // The segments of a line are made equal.  A domain with fewer tiles than SMs takes fewer lines per
 // tile: a pass over it lasts as long as one position's chain, whatever a tile holds.  Large units
-// leave about four tiles per resident block to single-tile units, which end the launch evenly.
+// leave about `tail` tiles per resident block to single-tile units, which end the launch evenly: 4
+// in FP32 (8 and 16 cost its streamed domains 2-5 %), 8 in FP64 (1001x573 Godunov 7.6 ms, against 9.0
+// with 4; the moving flow and the circular Sod within 1 %), 16 in an FP64 batch, whose domains end one
+// by one (16 uneven domains 159 ms, against 172 with 8, 179 with 4, 166 with 32).
 template <class T>
-void set_tile_axis(AxisGeom<T>& g, bool rows, int halo, int sms, int slots, int y_lines)
+void set_tile_axis(AxisGeom<T>& g, bool rows, int halo, int sms, int slots, int y_lines, int tail)
 {
     const int want = rows ? 1 : std::max(1, std::min(y_lines, g.nlines));
     const int longest = std::max(1, rows ? std::min(248, kTileBlock - 2 * halo) : kTileBlock / want / 8 * 8 - 2 * halo);
@@ -109,7 +112,7 @@ void set_tile_axis(AxisGeom<T>& g, bool rows, int halo, int sms, int slots, int 
     if (!rows && g.tile_scan)       // a large unit of columns lies in one segment
         g.tile_groups = (g.tile_groups + kTileUnit - 1) / kTileUnit * kTileUnit;
     const int64_t tiles = (int64_t)segs * g.tile_groups;
-    int64_t big = std::max<int64_t>(0, (tiles - 4 * (int64_t)slots) / kTileUnit);
+    int64_t big = std::max<int64_t>(0, (tiles - tail * (int64_t)slots) / kTileUnit);
     g.tile_big = (int)big;
     g.tile_units = (int)(big + (tiles - big * kTileUnit));
 }

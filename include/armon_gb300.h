@@ -83,8 +83,11 @@ typedef struct armon_solver_opts {
     int32_t precision;        /* 64: FP64 state and arithmetic (bit-exact with the reference);
                                  32: FP32 state and arithmetic, FP64 dt and conservation sums */
     int32_t cycles_per_graph; /* cycles captured per CUDA graph launch (0 = default, 16) */
-    int32_t seg_len;          /* cells per thread along the sweep axis (0 = automatic) */
-    int32_t block_lines;      /* lines (threads) per block (0 = automatic, 128) */
+    /* seg_len, block_lines and split_pass all 0 (default): the axis passes run in the tile form, one
+       thread per position (csrc/sweep_tile.cuh).  Any of them set selects the marches, one thread per
+       line segment.  Results are the same bits in every form. */
+    int32_t seg_len;          /* marches: cells per thread along the sweep axis (0 = automatic) */
+    int32_t block_lines;      /* marches: lines (threads) per block (0 = automatic, 128) */
     int32_t materialize_eos;  /* p, c, g of the real cells: written by every pass (1), by the last
                                  pass of each cycle (0), or (-1, default) computed from the last
                                  pass's input, which the other state set still holds, when the loop
@@ -94,17 +97,15 @@ typedef struct armon_solver_opts {
                                  arrays hold older values while cycles are still being issued
                                  (armon_solver_enqueue_cycles).  Split passes write them on the last
                                  pass in modes -1 and 0 (their cell half reads c). */
-    int32_t unit_order;       /* 0 (default): each pass launches its blocks longest first, by the time
-                                 each took in the previous cycle (results do not depend on it);
-                                 -1: in index order */
-    int32_t split_pass;       /* 0 (default): an FP64 solver holds a face buffer (3 x max((nx+5) ny,
-                                 (ny+5) nx) values) and runs each axis pass as two launches (face
-                                 fluxes, then the cell update: fewer values per thread, more warps
-                                 per SM) or as one fused launch (half the bytes), whichever its
-                                 tiling measurement finds faster (domains under 2^20 cells: split;
-                                 fused when the face buffer cannot be allocated); FP32 passes stay
-                                 fused.  1: split for either precision; -1: fused.  Results are the
-                                 same bits either way. */
+    int32_t unit_order;       /* marches: 0 (default): each pass launches its blocks longest first, by
+                                 the time each took in the previous cycle (results do not depend on
+                                 it); -1: in index order */
+    int32_t split_pass;       /* 1: marches, each axis pass as two launches (face fluxes through a face
+                                 buffer of 3 x max((nx+5) ny, (ny+5) nx) values, then the cell
+                                 update); -1: marches, one fused launch; 0: the tile form, or, when
+                                 seg_len or block_lines selects the marches, split passes in FP64 (or
+                                 what the tiling measurement finds faster; fused when the face buffer
+                                 cannot be allocated) and fused ones in FP32 */
     int32_t reuse;            /* 0 (default): along each line, a position whose whole input window
                                  (the cells, and faces, its results depend on) repeats the previous
                                  position's bit for bit stores the previous position's results
@@ -162,13 +163,13 @@ int armon_solver_conservation(armon_solver* s, double* mass, double* energy);
 /* Number of kernels the solver launched so far (diagnostics). */
 int64_t armon_solver_kernel_launches(armon_solver* s);
 
-/* The tiling of the axis pass per axis (X, Y): cells per thread along the axis and blocks per
- * launch.  Unless opts.seg_len fixes it, a domain of 2^20 cells or more gets the fastest of a few
+/* The tiling of the axis pass per axis (X, Y): cells per tile (or, for marches, per thread) along the
+ * axis and blocks per launch.  Unless opts.seg_len fixes it, a domain of 2^20 cells or more gets the fastest of a few
  * candidate tilings, each timed on real cycles of its first time loop (after 16 cycles with the
  * model's tiling, two cycles per candidate forwards and two backwards: results never depend on
  * the tiling), and cached per geometry for the process; smaller domains use the cost model. */
 int armon_solver_tiling(armon_solver* s, int32_t seg_len[2], int32_t blocks[2]);
-/* Lines (threads) per block of the fused pass: the caller's block_lines, or the measured choice. */
+/* Lines (threads) per block of a march: the caller's block_lines, or the measured choice. */
 int armon_solver_block_lines(const armon_solver* s);
 /* 1 while the time loop is still measuring candidate tilings on its cycles (domains of 2^20 cells
  * or more whose geometry this process has not measured yet; results never depend on the tiling). */
@@ -176,8 +177,8 @@ int armon_solver_tuning(const armon_solver* s);
 /* Cycles this solver has run with a candidate tiling of the tiling measurement so far (a cost cycle
  * and a timed cycle per candidate and visit). */
 int64_t armon_solver_measurement_cycles(const armon_solver* s);
-/* 1 when the axis passes run split (a face launch and a cell launch), 0 when fused: the caller's
- * split_pass, or the measured form when split_pass is 0 and the solver holds a face buffer. */
+/* 1 when the axis passes run split (a face launch and a cell launch), 0 when a pass is one launch
+ * (tiles, or fused marches). */
 int armon_solver_split_pass(const armon_solver* s);
 /* Forgets the tilings measured so far in this process (the next time loop of each geometry
  * measures again). */
@@ -190,15 +191,17 @@ typedef struct armon_batch armon_batch;
 typedef struct armon_batch_opts {
     int32_t precision;        /* 64 or 32: every domain of a batch has this precision */
     int32_t cycles_per_graph; /* cycles captured per CUDA graph launch (default 8) */
-    int32_t block_lines;      /* lines (threads) per block: a multiple of 32, at most 128 (default 128) */
-    int32_t seg_len;          /* cells per thread along the sweep axis for every domain (0 = scheduled) */
+    /* block_lines 128, seg_len, waves and split_pass 0 (default): passes in the tile form, as a
+       solver's.  Anything else selects the marches. */
+    int32_t block_lines;      /* marches: lines (threads) per block: a multiple of 32, at most 128 (default 128) */
+    int32_t seg_len;          /* marches: cells per thread along the sweep axis for every domain (0 = scheduled) */
     int64_t memory_budget;    /* bytes of domain state the batch may hold (0 = no limit) */
-    int32_t waves;            /* scheduled segments: block waves per launch to aim for (0 = autotuned) */
-    int32_t unit_order;       /* 0 (default): each pass launches the blocks of all domains longest
+    int32_t waves;            /* marches: block waves per launch the scheduled segments aim for (0 = autotuned) */
+    int32_t unit_order;       /* marches: 0 (default): each pass launches the blocks of all domains longest
                                  first, by the time each took in the previous cycle; -1: in index order */
-    int32_t split_pass;       /* as armon_solver_opts.split_pass: 0 (default) split FP64 passes into a
-                                 face launch and a cell launch (each domain then holds a face buffer,
-                                 counted by armon_batch_domain_bytes); 1: split; -1: fused */
+    int32_t split_pass;       /* as armon_solver_opts.split_pass; an FP64 domain holds a face buffer
+                                 (counted by armon_batch_domain_bytes) unless this is -1, for the
+                                 split marches that armon_batch_set_seg_len selects */
     int32_t reuse;            /* as armon_solver_opts.reuse: 0 (default) on, -1 off */
 } armon_batch_opts;
 
