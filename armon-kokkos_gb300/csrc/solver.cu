@@ -485,6 +485,8 @@ int finish_tuning(armon_solver* s)
         if (visits[i] < 2) continue;
         if (!have || total[i] < best_t) { best = i; best_t = total[i]; have = true; }
     }
+    // tiles: the usual columns unless the others win by more than two timed cycles differ
+    if (have && T.cand[0][3] == kTileForm && visits[0] >= 2 && total[0] < 1.03f * best_t) best = 0;
     const Tiling choice = ran && have ? T.cand[best] : model_tiling(s);
     const std::array<int, 9> key = T.key;
     end_tuning(s);

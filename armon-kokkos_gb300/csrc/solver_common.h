@@ -74,12 +74,13 @@ inline AxisTiling choose_segments(int n, int nlines, int block, int halo, int sm
 }
 
 // Threads of a tile (sweep_tile.cuh), and the columns of a Y tile.  More columns read longer stretches
-// of a row, fewer leave longer tiles and less halo: two of 120 positions (halo 6 %), three of 72 or
-// four of 56 (13 %).  FP64, bound by its arithmetic, takes two (a 2048x2048 moving flow, 24 cycles:
-// 45.9 ms, against 47.5 with three or four); FP32 three (48 small domains: 17.5 ms, against 18.8 with
-// two and 18.5 with four; large domains within 1 %).
+// of a row, fewer leave longer tiles and less halo: two of 120 positions (halo 6 %), four of 56 (13 %),
+// eight of 24 (25 %).  FP64, bound by its arithmetic, takes two (a 2048x2048 moving flow, 24 cycles:
+// 45.9 ms, against 47.5 with three or four); FP32, bound by its instructions and loads, eight (the
+// same flow, 15 cycles: 6.37 ms, against 6.44 with four and 6.67 with two; 48 small domains 17.1 ms,
+// against 18.4 and 18.8).
 constexpr int kTileBlock = 256;
-template <class T> constexpr int tile_y_lines() { return sizeof(T) == 8 ? 2 : 3; }
+template <class T> constexpr int tile_y_lines() { return sizeof(T) == 8 ? 2 : 8; }
 
 // The tiles of one axis.  A tile is `lines` lines by width = len + 2 halo positions, at most kTileBlock
 // threads.  Along rows (X) the positions are consecutive in memory, so a tile is as long as the block
@@ -107,7 +108,7 @@ void set_tile_axis(AxisGeom<T>& g, bool rows, int halo, int sms, int slots, int 
     g.tile_lines = std::max(1, std::min({rows ? fit : std::min(fit, want), g.nlines, spread}));
     g.tile_groups = (g.nlines + g.tile_lines - 1) / g.tile_lines;
     // worth a scan when a block has several tiles; the walls' positions may not overlap
-    g.tile_scan = (rows ? g.tile_lines == 1 : g.tile_lines * kTileUnit <= 32 && (g.tile_width + 7) / 8 * 8 * g.tile_lines <= kTileBlock) && g.n >= 32 &&
+    g.tile_scan = (rows ? g.tile_lines == 1 : g.tile_lines * kTileUnit <= 64 && (g.tile_width + 7) / 8 * 8 * g.tile_lines <= kTileBlock) && g.n >= 32 &&
                   (int64_t)segs * g.tile_groups >= 3 * (int64_t)slots;
     if (!rows && g.tile_scan)       // a large unit of columns lies in one segment
         g.tile_groups = (g.tile_groups + kTileUnit - 1) / kTileUnit * kTileUnit;

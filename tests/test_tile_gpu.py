@@ -25,7 +25,7 @@ def tile_axis(n, nlines, rows, halo, sms, slots, y_lines):
     spread = max(1, nlines * segs // sms)
     lines = max(1, min(fit if rows else min(fit, want), nlines, spread))
     groups = -(-nlines // lines)
-    scan = (lines == 1 if rows else lines * 8 <= 32 and -(-width // 8) * 8 * lines <= 256) and n >= 32 \
+    scan = (lines == 1 if rows else lines * 8 <= 64 and -(-width // 8) * 8 * lines <= 256) and n >= 32 \
         and segs * groups >= 3 * slots
     if not rows and scan:
         groups = -(-groups // 8) * 8
@@ -36,7 +36,7 @@ def tile_axis(n, nlines, rows, halo, sms, slots, y_lines):
 
 
 @pytest.mark.parametrize("halo", [2, 3, 4])
-@pytest.mark.parametrize("y_lines", [2, 3, 4])
+@pytest.mark.parametrize("y_lines", [2, 4, 8])
 def test_tiles_cover_each_cell_once_and_stay_in_the_ghosts(halo, y_lines):
     sizes = (1, 5, 17, 31, 32, 100, 119, 120, 121, 239, 240, 241, 247, 248, 249, 256, 300, 497, 1000)
     for n in sizes:
