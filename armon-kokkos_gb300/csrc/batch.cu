@@ -1,12 +1,12 @@
 // batch.cu -- many independent domains advanced together (include/armon_gb300.h, armon_batch_*).
 //
 // Every domain keeps its own state (two buffer sets, p/c/g, dt partials) in one allocation from
-// the batch's stream-ordered memory pool, and its own 48-byte step state in a slot of a device
-// array.  A pass over the batch is one launch of sweep_batch_kernel: the launch table lists the
-// running domains and the first grid block of each (enough blocks for its larger axis), so one
-// launch covers every domain, each with its own dt, time and cycle.  The table is rebuilt when
-// domains join or finish; cycles are captured in a CUDA graph per table.  The host reads all
-// step states back with one copy per graph batch.
+// the batch's stream-ordered memory pool, and its own 64-byte step state in a slot of a device
+// array.  A pass over the batch is one launch: in the tile form, tile_batch_kernel, whose resident
+// blocks are shared out to the running domains (rebuild_tiles); in marches, sweep_batch_kernel or its
+// split pair, whose launch table lists the first grid block of each domain.  Every domain keeps its
+// own dt, time and cycle.  The table is rebuilt when domains join or finish; cycles are captured in a
+// CUDA graph per table.  The host reads all step states back with one copy per graph batch.
 #include <algorithm>
 #include <array>
 #include <cstring>

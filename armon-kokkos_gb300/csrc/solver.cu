@@ -1,11 +1,12 @@
 // solver.cu -- the native solver: device-resident state, the fused time loop and its C ABI
 // (include/armon_gb300.h).
 //
-// One cycle = passes_per_cycle(splitting) axis passes, each one fused launch or a face and a cell
-// launch (the tiling measurement picks the form); the last one also reduces dt_CFL of the new
+// One cycle = passes_per_cycle(splitting) axis passes, each one launch in the tile form
+// (sweep_tile.cuh), or a march when the caller's options ask for one: one fused launch, or a face and a
+// cell launch.  The last one also reduces dt_CFL of the new
 // state and commits the cycle (time, cycle, dts) into the device StepState, so the host never
 // waits inside the loop.  Cycles are issued in batches captured in a CUDA graph;
-// after each batch the host reads the 48-byte state back to test the reference's loop condition
+// after each batch the host reads the 64-byte state back to test the reference's loop condition
 // (time < max_time && cycle < max_cycles).  Cycles issued past the end are no-ops on the device.
 #include <algorithm>
 #include <array>
@@ -295,7 +296,8 @@ int ensure_stage(armon_solver* s)
     return ARMON_OK;
 }
 
-// Tiling of a lone domain, measured on the caller's own cycles.  With the GPU to itself, the best
+// Tiling of a lone domain, measured on the caller's own cycles.  The tile form compares two widths of
+// its Y tiles.  For marches with the GPU to itself, the best
 // segment length depends on more than the cells a thread walks (how full the last wave of blocks
 // is, how many blocks share an SM, how unevenly the units cost -- fronts against fluid at rest --,
 // cache traffic), and so does the pass form (split passes keep the FP64 pipe busier where cells are

@@ -11,6 +11,18 @@
 // and only a stage's operands are alive at once, so more warps share an SM, a pass over a small
 // domain lasts as long as one position's chain, and both axes read consecutive addresses.
 //
+// What bounds it.  FP64 where every position is computed (2048x2048 moving flow): the FP64 pipe, 76 %
+// busy with ~106 operations a position on 24 warps per SM (a march's 8 to 12 warps left it 60-75 %
+// busy in each of two launches): 0.94 ms an X pass; 24 cycles 78.2 ms with marches, 45.9 ms now.  FP32
+// there: instruction issue, 70 % busy, 0.14 ms.  A uniform fluid with fronts (4096x4096 circular Sod):
+// a block's own chain of scan, stores and computed stretches (30 000 cycles each), three blocks per
+// SM; 0.38-0.45 ms a pass late in the run, against 1.1 ms.  Small domains: one position's ~3000
+// dependent instructions, 16 us a pass (96x64: 42 us a cycle, 546 us with marches).
+// Measured and dropped: 64 registers and four blocks per SM in FP64 (spills; +4 to +20 %), products on
+// the integer pipes (dense 5 % faster at best, fronts 15-40 % slower), the quotients of a stage in one
+// straight-line group (+7 to +10 %: more code), cells of the next unit asked for in L2 (+8 %),
+// batches of eight cells in a scan (+4 %).
+//
 // Tile geometry.  X pass: a tile is tile_lines rows by tile_width positions, thread = row * tile_width +
 // position, so a warp reads a stretch of a row.  Y pass: tile_lines columns by tile_width positions,
 // thread = position * tile_lines + column; the neighbours along the axis are tile_lines threads away.

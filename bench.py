@@ -270,7 +270,7 @@ def run_reference(args) -> None:
 
 # ---------------------------------------------------------------- parity against the oracle
 def parity(A, case, cycles: int, precision: int = 64) -> dict:
-    """The GPU solver (default options: measured tiling, longest-first dispatch, split passes, reuse)
+    """The GPU solver (default options: the tile form with measured tiling, reuse)
     against the strict oracle, cycle by cycle: max and L1 relative error per field after `cycles`
     cycles, and the largest relative difference of (current dt, next dt, time) over every cycle."""
     import numpy as np
@@ -399,7 +399,12 @@ def e2e_run(A, args, nx: int, prec: int, cycles: int, stream, ins: dict, outs: d
     return secs, nb, e0.elapsed_time(e1)
 
 
-def roofline(prec: int, cells: int, ms_per_cycle: float, split: bool) -> dict:
+def default_form(args, split_pass: int | None = None) -> bool:
+    """Whether the options leave the solver its default form, tiles (marches otherwise)."""
+    return args.seg_len <= 0 and args.block_lines <= 0 and (args.split_pass if split_pass is None else split_pass) == 0
+
+
+def roofline(prec: int, cells: int, ms_per_cycle: float, split: bool, tile: bool) -> dict:
     peak, peak_kind = measured_peaks()
     t_pass = ms_per_cycle / 1e3 / 2
     bpc = BYTES_PER_CELL_UPDATE if prec == 64 else BYTES_PER_CELL_UPDATE // 2
@@ -407,8 +412,9 @@ def roofline(prec: int, cells: int, ms_per_cycle: float, split: bool) -> dict:
     tname = "double" if prec == 64 else "float"
     kernel = ("armon::sweep_faces_kernel<%s,1,2,*> + armon::sweep_cells_kernel<%s,1,2,*> (one axis pass = a face "
               "launch and a cell launch)" % (tname, tname) if split else
+              "armon::tile_kernel<%s,1,2,true> (one launch = one axis pass)" % tname if tile else
               "armon::sweep_kernel<%s,1,2,*> (one launch = one axis pass)" % tname)
-    key = ("split_" if split else "fused_") + "traffic_bytes_per_cell_per_pass"
+    key = ("split_" if split else "tile_" if tile else "fused_") + "traffic_bytes_per_cell_per_pass"
     tr = profiled(key, prec)
     return {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
             "peak_source": peak_kind + " (MEASURED_PEAKS.json hbm_gbs, a STREAM-style copy)",
@@ -468,7 +474,7 @@ def run_gpu(args) -> None:
                "whole_run": {"value": whole, "unit": METRIC, "cycles": run_cycles,
                              "note": "every cycle of the whole run, from the initial state, on the device (CUDA events "
                                      "around begin_loop and the time loop of the e2e solve)"},
-               "roofline": roofline(prec, cells, ms_max / K, r["split"]),
+               "roofline": roofline(prec, cells, ms_max / K, r["split"], default_form(args)),
                "e2e": {"value": e2e_value, "unit": METRIC, "cycles": run_cycles,
                        "h2d_bytes_per_step": 4 * nb * 8 / run_cycles, "d2h_bytes_per_step": 5 * nb * 8 / run_cycles,
                        "seconds": e2e_s, "host_arrays": "FP64 (converted to the solver's precision inside the call)",
@@ -534,7 +540,7 @@ def fp32_line(A, args, stream) -> dict:
                            split_pass=r["split"], timed_cycles=[r["total"] - K, r["total"]],
                            tiling_measurement_cycles=r["measurement_cycles"],
                            tiling_measurement_cycles_timed=r["measured_in_window"]),
-            "roofline": roofline(32, cells, r["ms"] / K, r["split"]),
+            "roofline": roofline(32, cells, r["ms"] / K, r["split"], default_form(args, 0)),
             "accuracy": fp32_accuracy(A, nx, 100, args.graph) if args.accuracy_cycles > 0 else None,
             "gpu_launches": r["launches"], "clocks": r["clocks"]}
 
