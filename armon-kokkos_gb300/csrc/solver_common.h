@@ -107,8 +107,10 @@ void set_tile_axis(AxisGeom<T>& g, bool rows, int halo, int sms, int slots, int 
     const int spread = (int)std::max<int64_t>(1, (int64_t)g.nlines * segs / sms);
     g.tile_lines = std::max(1, std::min({rows ? fit : std::min(fit, want), g.nlines, spread}));
     g.tile_groups = (g.nlines + g.tile_lines - 1) / g.tile_lines;
-    // worth a scan when a block has several tiles; the walls' positions may not overlap
+    // worth a scan when a block has several tiles; the walls' positions may not overlap, and a stretch's
+    // first position is held in 23 bits
     g.tile_scan = (rows ? g.tile_lines == 1 : g.tile_lines * kTileUnit <= 64 && (g.tile_width + 7) / 8 * 8 * g.tile_lines <= kTileBlock) && g.n >= 32 &&
+                  g.n < (1 << 23) &&
                   (int64_t)segs * g.tile_groups >= 3 * (int64_t)slots;
     if (!rows && g.tile_scan)       // a large unit of columns lies in one segment
         g.tile_groups = (g.tile_groups + kTileUnit - 1) / kTileUnit * kTileUnit;

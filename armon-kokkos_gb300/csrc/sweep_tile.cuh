@@ -73,7 +73,7 @@ enum : int { kRunRho, kRunUa, kRunUo, kRunE, kRunP, kRunC, kRunOut, kRunWall = k
 // Consecutive owned positions of a line waiting to be computed.
 struct Stretch {
     int32_t line;
-    int32_t start_len;    // first position << 8 | positions (at most 248)
+    int32_t start_len;    // first position (below 2^23) << 8 | positions (at most 248)
 };
 
 template <class T>

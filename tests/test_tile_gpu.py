@@ -25,7 +25,7 @@ def tile_axis(n, nlines, rows, halo, sms, slots, y_lines):
     spread = max(1, nlines * segs // sms)
     lines = max(1, min(fit if rows else min(fit, want), nlines, spread))
     groups = -(-nlines // lines)
-    scan = (lines == 1 if rows else lines * 8 <= 64 and -(-width // 8) * 8 * lines <= 256) and n >= 32 \
+    scan = (lines == 1 if rows else lines * 8 <= 64 and -(-width // 8) * 8 * lines <= 256) and 32 <= n < 1 << 23 \
         and segs * groups >= 3 * slots
     if not rows and scan:
         groups = -(-groups // 8) * 8
