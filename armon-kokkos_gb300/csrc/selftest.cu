@@ -1,11 +1,14 @@
 // selftest.cu -- checks of the integer-pipe FP64 operations (softfp.cuh) against the FP64
-// instructions, on generated operands.  Exposed as armon_selftest_softfp for the test suite.
+// instructions, on generated operands (armon_selftest_softfp), and host entries to the tile form's index
+// arithmetic (armon_selftest_tile_*), for the test suite.
 #include <cstdint>
 #include <cstring>
 
 #include <cuda_runtime.h>
 
 #include "softfp.cuh"
+#include "solver_common.h"
+#include "sweep_tile.cuh"
 
 namespace {
 
@@ -308,6 +311,41 @@ int armon_selftest_add_host(uint64_t seed, int64_t n, uint64_t* out)
         }
     }
     return 0;
+}
+
+// The tiles that set_tile_axis gives an axis of n cells and nlines lines: out = len, width, lines, segs,
+// groups, scan, big, units.
+int armon_selftest_tile_axis(int32_t n, int32_t nlines, int32_t rows, int32_t halo, int32_t sms, int32_t slots,
+                             int32_t y_lines, int32_t tail, int32_t* out)
+{
+    armon::AxisGeom<double> g{};
+    g.n = n;
+    g.nlines = nlines;
+    armon::set_tile_axis(g, rows != 0, halo, sms, slots, y_lines, tail);
+    const int32_t v[8] = {g.tile_len, g.tile_width, g.tile_lines, g.tile_segs, g.tile_groups, g.tile_scan, g.tile_big,
+                          g.tile_units};
+    std::memcpy(out, v, sizeof(v));
+    return 0;
+}
+
+// The places of a block's threads (stretch, position in it, in) when the list holds `count` stretches of
+// `cells` cells each: place[3 t ..] for thread t.  Returns how many stretches the block takes.
+int armon_selftest_tile_pack(const int32_t* cells, int32_t count, int32_t halo, int32_t* place)
+{
+    int need[32], sum[32], total = 0, take = 0;
+    for (int j = 0; j < 32; j++) {
+        need[j] = j < count ? cells[j] + 2 * halo : 1 << 20;
+        sum[j] = total += need[j];
+        take += total <= armon::kTileThreads;
+    }
+    for (int t = 0; t < armon::kTileThreads; t++) {
+        int k, q;
+        const bool in = armon::pack_place(t, take, [&](int j) { return sum[j]; }, [&](int j) { return need[j]; }, k, q);
+        place[3 * t] = k;
+        place[3 * t + 1] = q;
+        place[3 * t + 2] = in;
+    }
+    return take;
 }
 
 // mode 0..6 (see operands) checks sfp::div against the hardware quotient; mode 100 checks lt,

@@ -56,7 +56,7 @@ namespace armon {
 constexpr int kTileThreads = 256;
 constexpr int kTileWarps = kTileThreads / 32;
 constexpr int kTileSlots = 15;
-constexpr int kTileList = 512;        // stretches the list can hold (at most 128 per scan, 16 left over)
+constexpr int kTileList = 512;        // stretches the list can hold (at most 128 per scan, 32 left over)
 
 #ifndef ARMON_TILE_MIN_BLOCKS
 #define ARMON_TILE_MIN_BLOCKS 3
@@ -100,6 +100,25 @@ struct TileShared {
     int claims;                       // states recorded so far
     int next[2];                      // [unit parity]: the block's next unit
 };
+
+// The place of thread tid among packed stretches: the first stretch whose threads (sum(j): those of the
+// stretches up to j) end past it, k, and its position there, q.  False for a thread that stands for
+// none: behind the `take` stretches that fit, or behind the last of all 32, which the search's five
+// steps also give k = 31 (32 stretches of fewer than eight threads leave such threads: a segment's
+// last few cells with a stencil reach of two or three).  sum and need are the block's shuffles, or arrays on the host.
+#pragma nv_exec_check_disable
+template <class Sum, class Need>
+__host__ __device__ __forceinline__ bool pack_place(int tid, int take, Sum sum, Need need, int& k, int& q)
+{
+    k = 0;
+    for (int o = 16; o > 0; o >>= 1) {
+        const int v = sum(k + o - 1);
+        if (v <= tid) k += o;
+    }
+    const int threads = need(k);
+    q = tid - (sum(k) - threads);
+    return k < take && q < threads;
+}
 
 // The tiles of one unit of one domain.  SCAN: its units may be scanned (AxisGeom::tile_scan); without it
 // the pass is its stages alone, half the code.
@@ -596,20 +615,15 @@ struct TilePass {
         }
         const int take = __popc(__ballot_sync(0xffffffffu, sum <= kTileThreads));
         if (!all && take == left && __shfl_sync(0xffffffffu, sum, take - 1) < kTileThreads * 3 / 4) return false;
-        // this thread's stretch: the first whose sum lies above its index
-        int k = 0;
-        for (int o = 16; o > 0; o >>= 1) {
-            const int v = __shfl_sync(0xffffffffu, sum, k + o - 1);
-            if (v <= tid) k += o;
-        }
+        int k;
+        p.in = pack_place(tid, take, [&](int j) { return __shfl_sync(0xffffffffu, sum, j); },
+                          [&](int j) { return __shfl_sync(0xffffffffu, need, j); }, k, p.q);
         const int line = __shfl_sync(0xffffffffu, s.line, k);
         const int sl = __shfl_sync(0xffffffffu, s.start_len, k);
         p.hint = -1;
-        p.q = tid - __shfl_sync(0xffffffffu, sum - need, k);
         p.width = (sl & 255) + 2 * H;
         p.t = (sl >> 8) - H + p.q;
         p.base = A.origin + (int64_t)line * A.geom[axis].lstride;
-        p.in = k < take;
         centre = (__shfl_sync(0xffffffffu, s.start_len, 0) & 255) / 2 + H;
         __syncthreads();         // before sh.head or the entries are written again
         if (tid == 0) sh.head = head + take;
