@@ -112,8 +112,8 @@ struct armon_batch {
     bool tile = true;             // passes in the tile form (sweep_tile.cuh), unless a domain fixes its segments
     bool tiled = true;            // the current table's form
     int* d_units = nullptr;       // tile form: units of each domain
+    TileCtl* d_ctl = nullptr;     // the tile launches' counters: the launch's, then a ticket per domain
     uint32_t* d_tickets = nullptr;
-    TileCtl* d_ctl = nullptr;
     TileHints<double>* d_hints = nullptr;   // per slot
     bool split = true;            // passes as a face launch and a cell launch (sweep_split.cuh)
     bool ordered = true;          // longest-first dispatch of each pass's blocks
@@ -254,7 +254,8 @@ int rebuild_tiles(armon_batch* b)
     CUDA_TRY(cudaMemcpyAsync(b->d_args, args.data(), nd * sizeof(SweepArgs<T>), cudaMemcpyHostToDevice, b->stream));
     CUDA_TRY(cudaMemcpyAsync(b->d_offsets, first.data(), (nd + 1) * sizeof(int), cudaMemcpyHostToDevice, b->stream));
     CUDA_TRY(cudaMemcpyAsync(b->d_units, units.data(), nd * sizeof(int), cudaMemcpyHostToDevice, b->stream));
-    CUDA_TRY(cudaMemsetAsync(b->d_tickets, 0, nd * sizeof(uint32_t), b->stream));
+    // on the stream of the launches that use them
+    CUDA_TRY(cudaMemsetAsync(b->d_ctl, 0, sizeof(TileCtl) + nd * sizeof(uint32_t), b->stream));
     CUDA_TRY(cudaStreamSynchronize(b->stream));   // the host vectors go out of scope
     return ARMON_OK;
 }
@@ -559,10 +560,9 @@ int armon_batch_create(const armon_batch_opts* opts, void* stream, armon_batch**
     if (e == cudaSuccess) e = cudaMalloc(&b->d_args, sizeof(SweepArgs<double>) * kMaxDomains);
     if (e == cudaSuccess) e = cudaMalloc(&b->d_offsets, sizeof(int) * (kMaxDomains + 1));
     if (e == cudaSuccess) e = cudaMalloc(&b->d_units, sizeof(int) * kMaxDomains);
-    if (e == cudaSuccess) e = cudaMalloc(&b->d_tickets, sizeof(uint32_t) * kMaxDomains + sizeof(TileCtl));
-    if (e == cudaSuccess) e = cudaMemset(b->d_tickets, 0, sizeof(uint32_t) * kMaxDomains + sizeof(TileCtl));
+    if (e == cudaSuccess) e = cudaMalloc(&b->d_ctl, sizeof(TileCtl) + sizeof(uint32_t) * kMaxDomains);
     if (e == cudaSuccess) e = cudaMalloc(&b->d_hints, sizeof(TileHints<double>) * kMaxDomains);
-    b->d_ctl = reinterpret_cast<TileCtl*>(b->d_tickets + kMaxDomains);
+    b->d_tickets = reinterpret_cast<uint32_t*>(b->d_ctl + 1);
     if (e != cudaSuccess) {
         armon_batch_destroy(b);
         return cuda_fail(e, "batch allocation");
@@ -586,7 +586,7 @@ void armon_batch_destroy(armon_batch* b)
     if (b->d_args) cudaFree(b->d_args);
     if (b->d_offsets) cudaFree(b->d_offsets);
     if (b->d_units) cudaFree(b->d_units);
-    if (b->d_tickets) cudaFree(b->d_tickets);
+    if (b->d_ctl) cudaFree(b->d_ctl);
     if (b->d_hints) cudaFree(b->d_hints);
     if (b->d_order) cudaFree(b->d_order);
     if (b->d_cost) cudaFree(b->d_cost);

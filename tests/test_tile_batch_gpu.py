@@ -1,0 +1,60 @@
+"""Batches and servers in the tile form (csrc/batch.cu): what their launches share is set up on their own
+stream."""
+import numpy as np
+import pytest
+
+import armon_gb300 as A
+from test_batch_gpu import small_domains, solo
+
+pytestmark = pytest.mark.gpu
+
+FIELDS = ("rho", "umat", "vmat", "Emat", "pmat")
+
+
+def busy_default_stream(torch):
+    """Some tens of milliseconds of ordinary work queued on the default stream."""
+    t = torch.ones(1 << 28, device="cuda")
+    for _ in range(100):
+        t.mul_(1.0)
+    return t
+
+
+@pytest.mark.parametrize("precision", [64, 32])
+def test_batch_created_while_the_default_stream_is_busy(precision):
+    torch = pytest.importorskip("torch")
+    specs = small_domains(6, seed=17)
+    refs = [solo(s, precision=precision) for s in specs]
+    states = [s.initial_state() for s in specs]
+    busy = busy_default_stream(torch)
+    with A.Batch(precision=precision, cycles_per_graph=4) as b:
+        ids = [b.add(s.params(), st) for s, st in zip(specs, states)]
+        assert b.run() == 0
+        for i, (ps, _, ref) in zip(ids, refs):
+            pb, st = b.state(i)
+            assert st == 0 and (pb.cycle, pb.time, pb.next_cycle_dt) == (ps.cycle, ps.time, ps.next_cycle_dt)
+            for k in FIELDS:
+                got = A.real_cells(b.params[i], b.download(i, k))
+                assert np.array_equal(got.view(np.int64), ref[k].view(np.int64)), k
+    torch.cuda.synchronize()
+    del busy
+
+
+def test_server_created_while_the_default_stream_is_busy():
+    torch = pytest.importorskip("torch")
+    specs = small_domains(6, seed=19)
+    refs = [solo(s, precision=64 if k % 2 else 32) for k, s in enumerate(specs)]
+    busy = busy_default_stream(torch)
+    with A.Server() as srv:
+        ids = [srv.submit(s.params(), 64 if k % 2 else 32, s.sod_interface()) for k, s in enumerate(specs)]
+        done = set()
+        while len(done) < len(ids):
+            srv.step()
+            while (r := srv.next_done()) is not None:
+                done.add(r)
+        for i, (ps, _, ref) in zip(ids, refs):
+            assert (srv.info(i).cycle, srv.info(i).time) == (ps.cycle, ps.time)
+            for k in FIELDS:
+                got = A.real_cells(srv.params[i], srv.download(i, k))
+                assert np.array_equal(got.view(np.int64), ref[k].view(np.int64)), k
+    torch.cuda.synchronize()
+    del busy
