@@ -260,9 +260,12 @@ int rebuild_tiles(armon_batch* b)
     return ARMON_OK;
 }
 
+// The launch table of the running domains.  The batch stays dirty until it is complete: a rebuild that
+// fails is made again before anything is launched.
 template <class T>
 int rebuild_t(armon_batch* b)
 {
+    b->dirty = true;
     b->table.clear();
     for (int i = 0; i < (int)b->doms.size(); i++)
         if (b->doms[i].used && !b->doms[i].done) b->table.push_back(i);
@@ -274,8 +277,11 @@ int rebuild_t(armon_batch* b)
         cudaGraphExecDestroy(b->graph);
         b->graph = nullptr;
     }
-    b->dirty = false;
-    if (tiled) return b->table.empty() ? ARMON_OK : rebuild_tiles<T>(b);
+    if (tiled) {
+        const int rc = b->table.empty() ? ARMON_OK : rebuild_tiles<T>(b);
+        b->dirty = rc != ARMON_OK;
+        return rc;
+    }
     if (b->blocks_per_sm == 0 && !b->table.empty())
         b->blocks_per_sm = b->split ? sweep_batch_split_blocks_per_sm(b->fp32, b->scheme, b->proj, b->o.block_lines)
                                     : sweep_batch_blocks_per_sm(b->fp32, b->scheme, b->proj, b->o.block_lines);
@@ -322,6 +328,7 @@ int rebuild_t(armon_batch* b)
                                  b->stream));
         CUDA_TRY(cudaStreamSynchronize(b->stream));   // the host vectors go out of scope
     }
+    b->dirty = false;
     return ARMON_OK;
 }
 

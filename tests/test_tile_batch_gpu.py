@@ -58,3 +58,31 @@ def test_server_created_while_the_default_stream_is_busy():
                 assert np.array_equal(got.view(np.int64), ref[k].view(np.int64)), k
     torch.cuda.synchronize()
     del busy
+
+
+@pytest.mark.parametrize("precision", [64, 32])
+def test_a_table_that_cannot_be_built_is_not_run(precision):
+    # one cell per thread needs more partial slots than a 512 x 512 domain holds: refused at every call, and
+    # the batch goes on as before once the segments are automatic again
+    big = A.Case(test="Sod_circ", scheme="GAD", projection="euler_2nd", nghost=5, nx=512, ny=512, cfl=0.6, max_cycles=20,
+                 max_time=1e9)
+    small = A.Case(**{**big.__dict__, "nx": 48, "ny": 64})
+    with A.Batch(precision=precision, cycles_per_graph=4) as b:
+        ids = [b.add(A.make_params(c)) for c in (big, small)]
+        b.run(cycle_limit=6)
+        b.set_seg_len(ids[0], 1)
+        for _ in range(2):
+            with pytest.raises(A.ArmonError) as e:
+                b.run(cycle_limit=4)
+            assert e.value.code == A.ERR_STATE
+        b.set_seg_len(ids[0], 0)
+        assert b.run() == 0
+        for i, c in zip(ids, (big, small)):
+            with A.Solver(c, precision=precision) as s:
+                s.init_test()
+                s.run()
+                p, q = b.state(i)[0], s.state()[0]
+                assert (p.cycle, p.time, p.next_cycle_dt) == (q.cycle, q.time, q.next_cycle_dt)
+                for k in FIELDS:
+                    got, ref = A.real_cells(b.params[i], b.download(i, k)), A.real_cells(s.params, s.download(k))
+                    assert np.array_equal(got.view(np.int64), ref.view(np.int64)), k
