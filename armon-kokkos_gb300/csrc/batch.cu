@@ -30,6 +30,7 @@ constexpr int kMaxDomains = 8192;
 // which tuning is worth a graph batch per candidate.
 constexpr int kWaves[] = {2, 4, 8, 16, 64};
 constexpr int kNumWaves = sizeof(kWaves) / sizeof(kWaves[0]);
+constexpr int kUntunedWaves = 8;
 constexpr int64_t kTuneMinCells = 1 << 21;
 
 struct Tuner {
@@ -102,7 +103,7 @@ struct armon_batch {
     std::vector<int> table;
     int total_blocks = 0;
     int blocks_per_sm = 0;        // of the batch kernel (0: not yet known)
-    int waves = 8;                // block waves per launch the schedule aims for
+    int waves = kUntunedWaves;    // marches: block waves per launch the schedule aims for
     Tuner tune;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     bool dirty = true;
@@ -273,6 +274,11 @@ int rebuild_t(armon_batch* b)
     for (int i : b->table) tiled = tiled && b->doms[i].seg_len <= 0;
     if (tiled != b->tiled) b->blocks_per_sm = 0;
     b->tiled = tiled;
+    if (tiled && b->tune.phase == 1) {
+        // the candidates are the marches': their timing starts again when the marches do
+        b->tune = Tuner{};
+        b->waves = kUntunedWaves;
+    }
     if (b->graph) {
         cudaGraphExecDestroy(b->graph);
         b->graph = nullptr;

@@ -86,3 +86,23 @@ def test_a_table_that_cannot_be_built_is_not_run(precision):
                 for k in FIELDS:
                     got, ref = A.real_cells(b.params[i], b.download(i, k)), A.real_cells(s.params, s.download(k))
                     assert np.array_equal(got.view(np.int64), ref.view(np.int64)), k
+
+
+def test_the_marches_candidates_are_not_timed_on_tile_passes():
+    # marches (one domain fixes its segments) start to time their schedule; tile passes end that
+    case = A.Case(test="Sod_circ", scheme="GAD", projection="euler_2nd", nghost=5, nx=1024, ny=1100, cfl=0.6, max_cycles=200,
+                  max_time=1e9)
+    with A.Batch(cycles_per_graph=4) as b:
+        ids = [b.add(A.make_params(c)) for c in (case, case, A.Case(**{**case.__dict__, "nx": 64}))]
+        b.run(cycle_limit=4)
+        untuned = b.schedule()[0]
+        b.set_seg_len(ids[2], 64)
+        b.run(cycle_limit=4)
+        assert b.schedule()[0] != untuned          # the first candidate
+        b.set_seg_len(ids[2], 0)
+        for _ in range(7):
+            b.run(cycle_limit=4)
+            assert b.schedule()[0] == untuned
+        assert all(b.state(i)[0].cycle == 36 for i in ids)
+        got = [A.real_cells(b.params[i], b.download(i, "rho")) for i in ids[:2]]
+        assert np.array_equal(got[0], got[1])
