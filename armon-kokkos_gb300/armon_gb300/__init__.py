@@ -468,7 +468,8 @@ class Batch:
         self.params.pop(i, None)
 
     def schedule(self) -> tuple[int, int]:
-        """(block waves per launch in use, blocks of the current launch table)."""
+        """(block waves per launch of the marches' schedule, which tile passes do not use; blocks of the
+        current launch table)."""
         w, n = C.c_int32(), C.c_int32()
         check(lib().armon_batch_schedule(self._h, C.byref(w), C.byref(n)))
         return w.value, n.value

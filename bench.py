@@ -577,7 +577,7 @@ def stratified(items: list, key, n: int) -> list:
 
 def batch_line(args, compact: bool) -> dict:
     """Configuration 3: 256 uneven domains (seeded), FP64, each to t = 0.15, all in one batch (one
-    launch per pass half over every domain, CUDA graphs), against the plain single-domain path (one
+    launch per pass over every domain, CUDA graphs), against the plain single-domain path (one
     solver per domain, one after another) on the same domains, or on a stratified sample of them."""
     import torch
 
@@ -607,7 +607,7 @@ def batch_line(args, compact: bool) -> dict:
 
         secs, clocks = sampled(go)
         launches = b.kernel_launches - launches0
-        waves, _ = b.schedule()
+        waves, blocks = b.schedule()
         work = 0
         for i, sp in zip(ids, specs):
             p, st = b.state(i)
@@ -619,15 +619,30 @@ def batch_line(args, compact: bool) -> dict:
             "config": {"workload": f"{len(specs)} uneven Sod-interface domains (seed 2024), sides in {{64..1024}}, "
                                    "GAD-minmod + euler_2nd, CFL 0.6, each to t = 0.15",
                        "domains": len(specs), "cells": sum(sp.nx * sp.ny for sp in specs), "cell_updates": work,
-                       "step": "the whole batch run to completion (one launch per pass half over every domain, "
-                               "8-cycle CUDA graphs)"},
+                       "step": "the whole batch run to completion (%s over every domain, 8-cycle CUDA graphs)"
+                               % ("one launch per pass" if batch_in_tiles(args) or args.split_pass < 0 else
+                                  "one launch per pass half")},
             "plain": {"value": plain_value, "seconds": plain_secs, "domains": len(sample),
                       "sample": ("a stratified sample by domain size (one domain from each of %d equal slices of the "
                                  "%d sorted by cells)" % (len(sample), len(specs))) if len(sample) < len(specs) else "all",
                       "path": "one Solver per domain, one after another (time loops only)"},
             "batched_over_plain": value / plain_value,
-            "schedule": {"waves": waves, "how": "autotuned online (CUDA-event timing of one graph batch per candidate)"},
+            "schedule": batch_schedule(args, waves, blocks),
             "gpu_launches": launches, "clocks": clocks}
+
+
+def batch_in_tiles(args) -> bool:
+    """Whether the options leave the batch its default form, tiles (marches otherwise)."""
+    return args.split_pass == 0 and (args.block_lines or 128) == 128
+
+
+def batch_schedule(args, waves: int, blocks: int) -> dict:
+    """What the batch's launches were shaped by: tile passes have no block waves."""
+    if batch_in_tiles(args):
+        return {"form": "tiles", "blocks": blocks, "how": "resident blocks shared out to the running domains by cells, "
+                                                          "units from each domain's ticket counter"}
+    return {"form": "marches", "waves": waves, "blocks": blocks,
+            "how": "autotuned online (CUDA-event timing of one graph batch per candidate)"}
 
 
 # ---------------------------------------------------------------- configuration 4: serving

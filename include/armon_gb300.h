@@ -267,8 +267,9 @@ int armon_batch_download(armon_batch* b, int32_t id, int which, double* host);
 /* Frees a domain's state (stream-ordered) and its handle. */
 int armon_batch_remove(armon_batch* b, int32_t id);
 
-/* The batch schedule in use: block waves per launch the segments aim for (autotuned unless fixed
- * by armon_batch_opts.waves or seg_len) and the blocks of the current launch table. */
+/* The batch schedule: the block waves per launch that the segments of marches aim for (autotuned
+ * unless fixed by armon_batch_opts.waves or seg_len; passes in the tile form have no waves, and
+ * leave the number that marches would start with) and the blocks of the current launch table. */
 int armon_batch_schedule(armon_batch* b, int32_t* waves, int32_t* blocks);
 
 int32_t armon_batch_size(armon_batch* b);                /* domains held */
