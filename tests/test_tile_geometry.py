@@ -39,6 +39,37 @@ def test_packed_threads_stay_in_their_stretches(halo, count):
         assert [tuple(p[:2]) for p in place[:len(want)]] == want
 
 
+@pytest.mark.parametrize("tail", [4, 8, 16])
+@pytest.mark.parametrize("halo", [2, 3, 4])
+@pytest.mark.parametrize("y_lines", [2, 4, 8])
+def test_tiles_cover_each_cell_once_and_fit_the_block(halo, y_lines, tail):
+    sizes = (1, 5, 17, 31, 32, 100, 119, 120, 121, 240, 247, 248, 249, 300, 757, 1000)
+    for n in sizes:
+        for nlines in (1, 2, 7, 33, 700):
+            for rows in (True, False):
+                for slots in (1, 40, 608):
+                    g = tile_axis(n, nlines, rows, halo, slots, y_lines, tail)
+                    assert g["width"] == g["len"] + 2 * halo and g["lines"] * g["width"] <= 256 and g["len"] < 256
+                    if rows:
+                        assert g["len"] <= 248        # 31 chunks of eight
+                    # every segment holds a cell, the last one's included; tiles past the lines are empty
+                    assert (g["segs"] - 1) * g["len"] < n <= g["segs"] * g["len"]
+                    assert (g["groups"] * g["lines"] >= nlines) and g["lines"] <= nlines
+                    tiles = g["segs"] * g["groups"]
+                    assert g["units"] == g["big"] + tiles - 8 * g["big"] and 0 <= 8 * g["big"] <= tiles
+                    if g["scan"]:
+                        assert n >= 32 and tiles >= 3 * slots
+                        if rows:
+                            assert g["lines"] == 1
+                        else:
+                            # a unit lies in one segment, and its columns' chunks in the block's threads
+                            assert g["groups"] % 8 == 0 and 8 * g["lines"] * -(-g["width"] // 8) <= 256
+                        # the list holds what a scan can add (runs two idle chunks apart) and what packing
+                        # leaves: 512 stretches
+                        chunks = -(-g["len"] // 8)
+                        assert 8 * g["lines"] * -(-chunks // 3) + 32 <= 512
+
+
 # scanned domains whose last segment along Y (FP32: eight columns a tile, FP64: two) or X is shorter than a
 # stretch of eight threads: reach 2 (Godunov, euler) with up to three cells, reach 3 with one
 SHORT = [
