@@ -113,6 +113,8 @@ struct armon_batch {
     bool tile = true;             // passes in the tile form (sweep_tile.cuh), unless a domain fixes its segments
     bool tiled = true;            // the current table's form
     int* d_units = nullptr;       // tile form: units of each domain
+    int* d_rest = nullptr;        // the domains that no block starts on
+    int nrest = 0;
     TileCtl* d_ctl = nullptr;     // the tile launches' counters: the launch's, then a ticket per domain
     uint32_t* d_tickets = nullptr;
     TileHints<double>* d_hints = nullptr;   // per slot
@@ -217,8 +219,8 @@ std::vector<std::array<int, 2>> schedule_segments(const armon_batch* b)
 int order_arrays(const armon_batch* b) { return b->npass * (b->split ? 2 : 1); }
 
 // The launch table of tile passes.  The resident blocks are shared out to the domains in proportion to
-// their cells (a domain of less than half a block's share gets none and is joined by blocks that
-// finish theirs); a domain's tiles are cut as if it had that share of the GPU to itself.
+// their cells (a domain of less than half a block's share gets none and is dealt to a block that has
+// finished its own); a domain's tiles are cut as if it had that share of the GPU to itself.
 template <class T>
 int rebuild_tiles(armon_batch* b)
 {
@@ -230,7 +232,6 @@ int rebuild_tiles(armon_batch* b)
     std::vector<SweepArgs<T>> args(nd);
     std::vector<int> first(nd + 1, 0), units(nd, 0);
     double seen = 0;
-    int64_t all = 0;
     for (size_t k = 0; k < nd; k++) {
         Dom& d = b->doms[b->table[k]];
         const int whole[2] = {d.p.nx, d.p.ny};
@@ -246,15 +247,22 @@ int rebuild_tiles(armon_batch* b)
         }
         seen += share;
         first[k + 1] = std::min((int)std::lround(slots * seen), first[k] + units[k]);
-        all += units[k];
     }
     // at least one block, and no more than there are units
     if (first[nd] == 0)
         for (size_t k = 1; k <= nd; k++) first[k] = 1;
     b->total_blocks = first[nd];
+    // the domains without blocks, the ones with most units first
+    std::vector<int> rest;
+    for (size_t k = 0; k < nd; k++)
+        if (first[k + 1] == first[k]) rest.push_back((int)k);
+    std::stable_sort(rest.begin(), rest.end(), [&](int i, int j) { return units[i] > units[j]; });
+    b->nrest = (int)rest.size();
     CUDA_TRY(cudaMemcpyAsync(b->d_args, args.data(), nd * sizeof(SweepArgs<T>), cudaMemcpyHostToDevice, b->stream));
     CUDA_TRY(cudaMemcpyAsync(b->d_offsets, first.data(), (nd + 1) * sizeof(int), cudaMemcpyHostToDevice, b->stream));
     CUDA_TRY(cudaMemcpyAsync(b->d_units, units.data(), nd * sizeof(int), cudaMemcpyHostToDevice, b->stream));
+    if (!rest.empty())
+        CUDA_TRY(cudaMemcpyAsync(b->d_rest, rest.data(), rest.size() * sizeof(int), cudaMemcpyHostToDevice, b->stream));
     // on the stream of the launches that use them
     CUDA_TRY(cudaMemsetAsync(b->d_ctl, 0, sizeof(TileCtl) + nd * sizeof(uint32_t), b->stream));
     CUDA_TRY(cudaStreamSynchronize(b->stream));   // the host vectors go out of scope
@@ -399,10 +407,10 @@ int enqueue_direct(armon_batch* b, int n)
             if (b->tiled) {
                 const cudaError_t e =
                     b->fp32 ? launch_sweep_tile_batch((const SweepArgs<float>*)b->d_args, b->d_offsets, b->d_units,
-                                                      b->d_tickets, nd, k, b->d_ctl, b->scheme, b->proj, last,
+                                                      b->d_rest, b->nrest, b->d_tickets, nd, k, b->d_ctl, b->scheme, b->proj, last,
                                                       b->total_blocks, b->stream)
                             : launch_sweep_tile_batch((const SweepArgs<double>*)b->d_args, b->d_offsets, b->d_units,
-                                                      b->d_tickets, nd, k, b->d_ctl, b->scheme, b->proj, last,
+                                                      b->d_rest, b->nrest, b->d_tickets, nd, k, b->d_ctl, b->scheme, b->proj, last,
                                                       b->total_blocks, b->stream);
                 if (e != cudaSuccess) return cuda_fail(e, "batch tile launch");
                 b->launches++;
@@ -573,6 +581,7 @@ int armon_batch_create(const armon_batch_opts* opts, void* stream, armon_batch**
     if (e == cudaSuccess) e = cudaMalloc(&b->d_args, sizeof(SweepArgs<double>) * kMaxDomains);
     if (e == cudaSuccess) e = cudaMalloc(&b->d_offsets, sizeof(int) * (kMaxDomains + 1));
     if (e == cudaSuccess) e = cudaMalloc(&b->d_units, sizeof(int) * kMaxDomains);
+    if (e == cudaSuccess) e = cudaMalloc(&b->d_rest, sizeof(int) * kMaxDomains);
     if (e == cudaSuccess) e = cudaMalloc(&b->d_ctl, sizeof(TileCtl) + sizeof(uint32_t) * kMaxDomains);
     if (e == cudaSuccess) e = cudaMalloc(&b->d_hints, sizeof(TileHints<double>) * kMaxDomains);
     b->d_tickets = reinterpret_cast<uint32_t*>(b->d_ctl + 1);
@@ -599,6 +608,7 @@ void armon_batch_destroy(armon_batch* b)
     if (b->d_args) cudaFree(b->d_args);
     if (b->d_offsets) cudaFree(b->d_offsets);
     if (b->d_units) cudaFree(b->d_units);
+    if (b->d_rest) cudaFree(b->d_rest);
     if (b->d_ctl) cudaFree(b->d_ctl);
     if (b->d_hints) cudaFree(b->d_hints);
     if (b->d_order) cudaFree(b->d_order);

@@ -37,6 +37,8 @@ struct StepState {
 // Counters of a tile launch, shared by its blocks; the last block to finish leaves them zero.
 struct TileCtl {
     uint32_t ticket, arrived;
+    uint32_t dealt;                 // batches: domains of the list of small ones handed out
+    uint32_t reserved;              // (what follows is aligned to 8 bytes)
 };
 
 // Tiles of a large unit (sweep_tile.cuh).

@@ -41,13 +41,14 @@ cudaError_t launch_sweep_tile(const SweepArgs<double>& a, TileCtl* ctl, int sche
                               cudaStream_t st);
 cudaError_t launch_sweep_tile(const SweepArgs<float>& a, TileCtl* ctl, int scheme, int proj, bool last, int grid,
                               cudaStream_t st);
-// The same over many domains (doms, first, units, tickets: device arrays; tickets start as zeros and
-// are left so): domain d has units[d] units and blocks [first[d], first[d + 1]) to begin with.
-cudaError_t launch_sweep_tile_batch(const SweepArgs<double>* doms, const int* first, const int* units, uint32_t* tickets,
-                                    int ndom, int pass, TileCtl* ctl, int scheme, int proj, bool last, int grid,
+// The same over many domains (doms, first, units, rest, tickets: device arrays; tickets start as zeros
+// and are left so): domain d has units[d] units and blocks [first[d], first[d + 1]) to begin with; rest
+// lists the nrest domains without blocks, in the order they are taken up.
+cudaError_t launch_sweep_tile_batch(const SweepArgs<double>* doms, const int* first, const int* units, const int* rest,
+                                    int nrest, uint32_t* tickets, int ndom, int pass, TileCtl* ctl, int scheme, int proj, bool last, int grid,
                                     cudaStream_t st);
-cudaError_t launch_sweep_tile_batch(const SweepArgs<float>* doms, const int* first, const int* units, uint32_t* tickets,
-                                    int ndom, int pass, TileCtl* ctl, int scheme, int proj, bool last, int grid,
+cudaError_t launch_sweep_tile_batch(const SweepArgs<float>* doms, const int* first, const int* units, const int* rest,
+                                    int nrest, uint32_t* tickets, int ndom, int pass, TileCtl* ctl, int scheme, int proj, bool last, int grid,
                                     cudaStream_t st);
 int sweep_tile_batch_blocks_per_sm(bool fp32, int scheme, int proj);
 // Blocks of the tile pass resident on one SM.

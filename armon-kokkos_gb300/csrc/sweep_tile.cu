@@ -40,11 +40,12 @@ int tile_blocks_t(int scheme, int proj)
 }
 
 template <class T>
-cudaError_t launch_tile_batch_t(const SweepArgs<T>* doms, const int* first, const int* units, uint32_t* tickets, int ndom,
-                                int pass, TileCtl* ctl, int scheme, int proj, bool last, int grid, cudaStream_t st)
+cudaError_t launch_tile_batch_t(const SweepArgs<T>* doms, const int* first, const int* units, const int* rest, int nrest,
+                                uint32_t* tickets, int ndom, int pass, TileCtl* ctl, int scheme, int proj, bool last, int grid, cudaStream_t st)
 {
 #define ARMON_TB(S, P) \
-    tile_batch_kernel<T, S, P><<<grid, kTileThreads, 0, st>>>(doms, first, units, tickets, ndom, pass, ctl, last ? 1 : 0)
+    tile_batch_kernel<T, S, P><<<grid, kTileThreads, 0, st>>>(doms, first, units, rest, nrest, tickets, ndom, pass, ctl, \
+                                                         last ? 1 : 0)
     if (scheme == 1) {
         if (proj == 2) ARMON_TB(1, 2); else ARMON_TB(1, 1);
     } else {
@@ -82,18 +83,18 @@ cudaError_t launch_sweep_tile(const SweepArgs<float>& a, TileCtl* ctl, int schem
     return launch_tile_t<float>(a, ctl, scheme, proj, last, grid, st);
 }
 
-cudaError_t launch_sweep_tile_batch(const SweepArgs<double>* doms, const int* first, const int* units, uint32_t* tickets,
-                                    int ndom, int pass, TileCtl* ctl, int scheme, int proj, bool last, int grid,
+cudaError_t launch_sweep_tile_batch(const SweepArgs<double>* doms, const int* first, const int* units, const int* rest,
+                                    int nrest, uint32_t* tickets, int ndom, int pass, TileCtl* ctl, int scheme, int proj, bool last, int grid,
                                     cudaStream_t st)
 {
-    return launch_tile_batch_t<double>(doms, first, units, tickets, ndom, pass, ctl, scheme, proj, last, grid, st);
+    return launch_tile_batch_t<double>(doms, first, units, rest, nrest, tickets, ndom, pass, ctl, scheme, proj, last, grid, st);
 }
 
-cudaError_t launch_sweep_tile_batch(const SweepArgs<float>* doms, const int* first, const int* units, uint32_t* tickets,
-                                    int ndom, int pass, TileCtl* ctl, int scheme, int proj, bool last, int grid,
+cudaError_t launch_sweep_tile_batch(const SweepArgs<float>* doms, const int* first, const int* units, const int* rest,
+                                    int nrest, uint32_t* tickets, int ndom, int pass, TileCtl* ctl, int scheme, int proj, bool last, int grid,
                                     cudaStream_t st)
 {
-    return launch_tile_batch_t<float>(doms, first, units, tickets, ndom, pass, ctl, scheme, proj, last, grid, st);
+    return launch_tile_batch_t<float>(doms, first, units, rest, nrest, tickets, ndom, pass, ctl, scheme, proj, last, grid, st);
 }
 
 int sweep_tile_batch_blocks_per_sm(bool fp32, int scheme, int proj)

@@ -944,6 +944,7 @@ __device__ __forceinline__ bool tile_arrive(TileCtl* ctl)
         if (is_last) {
             ctl->ticket = 0;
             ctl->arrived = 0;
+            ctl->dealt = 0;
             __threadfence();
         }
     }
@@ -999,11 +1000,18 @@ tile_kernel(const __grid_constant__ SweepArgs<T> A, TileCtl* ctl, int last)
 // Many independent domains in one launch (batch.cu).  Blocks [first[d], first[d + 1]) start on domain d,
 // in proportion to its cells, so that a block keeps the states of one domain; a domain's units beyond
 // its blocks' first ones come from its own ticket counter.  A block that finds its domain's units
-// taken joins the domain with the most units left.  The last block to finish commits every domain.
+// taken is dealt the next of the domains that no block started on (`rest`, `nrest` of them), and when
+// those are all under way joins the domain with the most units left, blocks starting their search
+// apart so that domains with equally many left get one each.  The last block to finish commits every domain.
+// A small domain is a few units, so with thousands of them the search would be most of a pass, and
+// blocks that search at once would find the same domain: 8000 domains of 16 to 32 cells a side, 40
+// cycles, take 40 ms in FP32 (190 in FP64), against 1238 (1162) when every domain was searched for and
+// 80 (518) with marches.
 template <class T, int SCHEME, int PROJ>
 __global__ void __launch_bounds__(kTileThreads, tile_min_blocks<T>())
 tile_batch_kernel(const SweepArgs<T>* __restrict__ doms, const int* __restrict__ first, const int* __restrict__ units,
-                  uint32_t* __restrict__ tickets, int ndom, int pass, TileCtl* ctl, int last)
+                  const int* __restrict__ rest, int nrest, uint32_t* __restrict__ tickets, int ndom, int pass, TileCtl* ctl,
+                  int last)
 {
     __shared__ TileShared<T> sh;
     __shared__ __align__(16) SweepArgs<T> sA;
@@ -1036,20 +1044,35 @@ tile_batch_kernel(const SweepArgs<T>* __restrict__ doms, const int* __restrict__
                 atomicMax(ticket, (uint32_t)total);      // nothing to do here: no block joins it
             }
         }
-        // the domain with the most units left
+        // the next domain of the list
         __syncthreads();
-        if (tid == 0) pick = 0;
-        __syncthreads();
-        unsigned long long best = 0;
-        for (int k = tid; k < ndom; k += kTileThreads) {
-            const int left = units[k] - (first[k + 1] - first[k]) - (int)min(__ldcg(&tickets[k]), 0x3fffffffu);
-            if (left > 0) best = max(best, (unsigned long long)left << 32 | (unsigned)k);
+        int dealt = nrest;
+        if (nrest > 0) {
+            if (tid == 0) pick = __ldcg(&ctl->dealt) < (uint32_t)nrest ? atomicAdd(&ctl->dealt, 1u) : (uint32_t)nrest;
+            __syncthreads();
+            dealt = (int)pick;
+            __syncthreads();
         }
-        if (best != 0) atomicMax(&pick, best);
-        __syncthreads();
-        if (pick == 0) break;
-        d = (int)(uint32_t)pick;
-        __syncthreads();
+        if (dealt < nrest) {
+            d = rest[dealt];
+        } else {
+            // the domain with the most units left, the first from `from` on among equals
+            const int from = (int)((uint64_t)blockIdx.x * ndom / gridDim.x);
+            if (tid == 0) pick = 0;
+            __syncthreads();
+            unsigned long long best = 0;
+            for (int k = tid; k < ndom; k += kTileThreads) {
+                const int left = units[k] - (first[k + 1] - first[k]) - (int)min(__ldcg(&tickets[k]), 0x3fffffffu);
+                const int behind = k >= from ? k - from : k + ndom - from;
+                if (left > 0) best = max(best, (unsigned long long)left << 32 | (unsigned)(ndom - behind));
+            }
+            if (best != 0) atomicMax(&pick, best);
+            __syncthreads();
+            if (pick == 0) break;
+            d = from + ndom - (int)(uint32_t)pick;
+            if (d >= ndom) d -= ndom;
+            __syncthreads();
+        }
         if (tid == 0) pick = atomicAdd(&tickets[d], 1u);
         __syncthreads();
         u = first[d + 1] - first[d] + (int)(uint32_t)pick;

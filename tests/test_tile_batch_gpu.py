@@ -106,3 +106,32 @@ def test_the_marches_candidates_are_not_timed_on_tile_passes():
         assert all(b.state(i)[0].cycle == 36 for i in ids)
         got = [A.real_cells(b.params[i], b.download(i, "rho")) for i in ids[:2]]
         assert np.array_equal(got[0], got[1])
+
+
+@pytest.mark.parametrize("precision", [64, 32])
+def test_many_small_domains_and_a_large_one_match_solo(precision):
+    # more domains than the launch has blocks, most of them dealt out, one that all blocks join in the end, and
+    # a few that end before the others; every distinct size is compared
+    def case(nx, ny, cycles):
+        return A.Case(test="Sod_circ", scheme="GAD", projection="euler_2nd", nghost=5, nx=nx, ny=ny, cfl=0.6,
+                      max_cycles=cycles, max_time=1e9)
+
+    kinds = [case(16, 16, 12), case(17, 40, 9), case(33, 16, 12), case(90, 21, 12), case(700, 650, 12)]
+    order = [k % 4 for k in range(1300)]
+    order[801] = 4
+    refs = []
+    for c in kinds:
+        with A.Solver(c, precision=precision) as s:
+            s.init_test()
+            s.run()
+            p, _ = s.state()
+            refs.append(((p.cycle, p.time, p.next_cycle_dt), {k: A.real_cells(s.params, s.download(k)) for k in FIELDS}))
+    with A.Batch(precision=precision, cycles_per_graph=4) as b:
+        ids = [b.add(A.make_params(kinds[k])) for k in order]
+        assert b.run() == 0
+        for n, (i, k) in enumerate(zip(ids, order)):
+            p, st = b.state(i)
+            assert st == 0 and (p.cycle, p.time, p.next_cycle_dt) == refs[k][0], n
+            for f in FIELDS if n % 20 < 4 or k == 4 else ("rho",):
+                got = A.real_cells(b.params[i], b.download(i, f))
+                assert np.array_equal(got.view(np.int64), refs[k][1][f].view(np.int64)), (n, f)
