@@ -242,7 +242,7 @@ int rebuild_tiles(armon_batch* b)
         for (int axis = 0; axis < 2; axis++) {
             set_tile_axis(args[k].geom[axis], axis == 0, stencil_reach(&d.p),
                           std::max(1, (int)std::lround(b->sm_count * share)),
-                          std::max(1, (int)std::lround(slots * share)), tile_y_lines<T>(), b->fp32 ? 4 : 16);
+                          std::max(1, (int)std::lround(slots * share)), tile_y_lines<T>(), b->fp32 ? 4 : 16, true);
             units[k] = std::max(units[k], args[k].geom[axis].tile_units);
         }
         seen += share;

@@ -316,16 +316,25 @@ int armon_selftest_add_host(uint64_t seed, int64_t n, uint64_t* out)
 // The tiles that set_tile_axis gives an axis of n cells and nlines lines: out = len, width, lines, segs,
 // groups, scan, big, units.
 int armon_selftest_tile_axis(int32_t n, int32_t nlines, int32_t rows, int32_t halo, int32_t sms, int32_t slots,
-                             int32_t y_lines, int32_t tail, int32_t* out)
+                             int32_t y_lines, int32_t tail, int32_t scan, int32_t* out)
 {
     armon::AxisGeom<double> g{};
     g.n = n;
     g.nlines = nlines;
-    armon::set_tile_axis(g, rows != 0, halo, sms, slots, y_lines, tail);
+    armon::set_tile_axis(g, rows != 0, halo, sms, slots, y_lines, tail, scan != 0);
     const int32_t v[8] = {g.tile_len, g.tile_width, g.tile_lines, g.tile_segs, g.tile_groups, g.tile_scan, g.tile_big,
                           g.tile_units};
     std::memcpy(out, v, sizeof(v));
     return 0;
+}
+
+// Whether a lone domain of nx by ny cells is scanned by default.
+int armon_selftest_scan_default(int32_t nx, int32_t ny, int32_t precision)
+{
+    armon_params p{};
+    p.nx = nx;
+    p.ny = ny;
+    return precision == 32 ? armon::scan_default<float>(p) : armon::scan_default<double>(p);
 }
 
 // The places of a block's threads (stretch, position in it, in) when the list holds `count` stretches of

@@ -65,7 +65,7 @@ struct armon_solver {
         size_t pos = 0;             // next entry of seq
         bool warm = true;           // the entry's unit-cost cycle comes next, then its timed cycle
         std::vector<cudaEvent_t> ev;
-        std::array<int, 9> key{};
+        std::array<int, 10> key{};
     } tune;
     int64_t issued = 0;             // cycles issued since begin_loop
     int64_t cycle0 = 0;             // the cycle count at begin_loop
@@ -81,6 +81,9 @@ struct armon_solver {
     bool tile = false;              // each pass in the tile form (sweep_tile.cuh)
     bool default_tile = false;
     int tile_lines = 0;             // columns of a Y tile (0: the default)
+    int tile_scan = 0;              // 1, -1: units are, are not scanned (0: scan_default)
+    int source = 0;                 // what the loop started from: 1 + test after init_test, 0: the caller's arrays
+    bool from_test = false;         // the arrays hold init_test's state
     int tile_per_sm = 0;            // blocks of the tile kernel resident on an SM
     void* d_faces = nullptr;        // 3 * face_stride values
     int64_t face_stride = 0;
@@ -127,7 +130,8 @@ void fill_geom(armon_solver* s, SweepArgs<T>& a)
         int units = 1;
         for (int axis = 0; axis < 2; axis++) {
             set_tile_axis(a.geom[axis], axis == 0, stencil_reach(&s->p), s->sm_count, slots,
-                          s->tile_lines > 0 ? s->tile_lines : tile_y_lines<T>(), s->fp32 ? 4 : 8);
+                          s->tile_lines > 0 ? s->tile_lines : tile_y_lines<T>(), s->fp32 ? 4 : 8,
+                          s->tile_scan != 0 ? s->tile_scan > 0 : scan_default<T>(s->p));
             units = std::max(units, a.geom[axis].tile_units);
         }
         s->grid = std::min(slots, units);
@@ -297,27 +301,30 @@ int ensure_stage(armon_solver* s)
 }
 
 // Tiling of a lone domain, measured on the caller's own cycles.  The tile form compares two widths of
-// its Y tiles.  For marches with the GPU to itself, the best
-// segment length depends on more than the cells a thread walks (how full the last wave of blocks
-// is, how many blocks share an SM, how unevenly the units cost -- fronts against fluid at rest --,
-// cache traffic), and so does the pass form (split passes keep the FP64 pipe busier where cells are
-// computed, fused ones move half the bytes where runs are streamed), so the time loop times a few
-// candidates -- the model's segments and segments aiming at 1, 2, 3, 4, 6 and 8 waves of resident
-// blocks (FP32 also 12 and 16), for each form the solver can run (a solver holding a face buffer runs both) and for
-// blocks of 128 lines (also of 32 when the caller fixed it) -- keeps the fastest and caches it per
-// geometry for the process.  Results never depend on the tiling or the form, so the candidates run
-// the loop's real cycles: after kTuneDelay cycles with the model's tiling (the fronts form), each
-// candidate runs one cycle that records its units' costs (for longest-first dispatch) and one timed
-// cycle, the list forwards, then the four fastest again backwards, so that a cost drifting with the
-// flow weighs alike on the finalists.  The loop pays only the difference between the candidates and
-// the best, a few cycles' worth.  A loop that ends before the measurement does keeps the model's
-// tiling and caches nothing.  Domains under 2^20 cells, single-pass splittings and a caller-fixed
-// seg_len are left to the model.
+// its Y tiles, or, in FP32 below 2^23 cells, units scanned and not: which is faster there depends on how
+// much of the domain is at rest (2048x2048, 60 cycles: circular Sod 22 ms scanned and 17.0 computed, Sedov
+// 8.4 and 17).
+// For marches with the GPU to itself, the best segment length depends on more than the cells a thread
+// walks (how full the last wave of blocks is, how many blocks share an SM, how unevenly the units cost
+// -- fronts against fluid at rest --, cache traffic), and so does the pass form (split passes keep the
+// FP64 pipe busier where cells are computed, fused ones move half the bytes where runs are streamed),
+// so the time loop times a few candidates -- the model's segments and segments aiming at 1, 2, 3, 4, 6
+// and 8 waves of resident blocks (FP32 also 12 and 16), for each form the solver can run (a solver
+// holding a face buffer runs both) and for blocks of 128 lines (also of 32 when the caller fixed it)
+// -- keeps the fastest and caches it per geometry, and per test problem or for the caller's own
+// states, for the process.
+// Results never depend on the tiling or the form, so the candidates run the loop's real cycles: after
+// kTuneDelay cycles with the model's tiling (the fronts form), each candidate runs one cycle that
+// records its units' costs (for longest-first dispatch) and one timed cycle, the list forwards, then
+// the four fastest again backwards, so that a cost drifting with the flow weighs alike on the
+// finalists.  The loop pays only the difference between the candidates and the best, a few cycles'
+// worth.  A loop that ends before the measurement does keeps the model's tiling and caches nothing.
+// Domains under 2^20 cells, single-pass splittings and a caller-fixed seg_len are left to the model.
 // segment length X, segment length Y, block lines, form (0 fused, 1 split); or for tiles (form
-// kTileForm): 0, columns of a Y tile, block lines, form
+// kTileForm): scan (armon_solver::tile_scan), columns of a Y tile, block lines, form
 using Tiling = std::array<int, 4>;
 constexpr int kTileForm = 2;
-std::map<std::array<int, 9>, Tiling> g_tilings;
+std::map<std::array<int, 10>, Tiling> g_tilings;
 std::mutex g_tilings_mu;
 constexpr int kTuneDelay = 16;
 constexpr size_t kTuneFinalists = 4;
@@ -346,21 +353,23 @@ int ensure_partials(armon_solver* s)
 
 int apply_tiling(armon_solver* s, const Tiling& t)
 {
-    s->tuned_seg[0] = t[0];
-    s->tuned_seg[1] = t[1];
     s->block = t[2];
     s->tile = t[3] == kTileForm;
-    if (s->tile) s->tile_lines = t[1];
+    s->tuned_seg[0] = s->tile ? 0 : t[0];
+    s->tuned_seg[1] = s->tile ? 0 : t[1];
+    s->tile_scan = s->tile ? t[0] : 0;
+    s->tile_lines = s->tile ? t[1] : 0;
     s->split = t[3] == 1 && s->d_faces != nullptr;
     int rc = refill(s);
     return rc != ARMON_OK ? rc : ensure_partials(s);
 }
 
-std::array<int, 9> tiling_key(const armon_solver* s)
+std::array<int, 10> tiling_key(const armon_solver* s)
 {
     const armon_params& p = s->p;
     return {p.nx, p.ny, s->fp32 ? 32 : 64, p.scheme, p.projection, p.axis_splitting, s->o.block_lines,
-            (s->o.split_pass + 1) | (s->d_faces ? 4 : 0) | (s->o.reuse >= 0 ? 8 : 0), s->ordered ? 1 : 0};
+            (s->o.split_pass + 1) | (s->d_faces ? 4 : 0) | (s->o.reuse >= 0 ? 8 : 0), s->ordered ? 1 : 0,
+            s->source};
 }
 
 // the cost model's tiling in the solver's default form
@@ -378,11 +387,20 @@ void end_tuning(armon_solver* s)
 // Called by begin_loop: the cached tiling of this geometry, or the measurement's set-up.
 int start_tuning(armon_solver* s)
 {
+    const bool tried = s->tune.active && s->tune.delay == 0;     // a candidate is in use
     end_tuning(s);
+    const int source = s->from_test ? 1 + s->p.test : 0;
+    s->from_test = false;
+    if (tried || (s->tuned && source != s->source)) {
+        s->tuned = false;
+        const int rc = apply_tiling(s, model_tiling(s));
+        if (rc != ARMON_OK) return rc;
+    }
+    s->source = source;
     if (s->tuned || s->o.seg_len > 0 || s->npass < 2) return ARMON_OK;
     const armon_params& p = s->p;
     if ((int64_t)p.nx * p.ny < (1 << 20)) return ARMON_OK;
-    const std::array<int, 9> key = tiling_key(s);
+    const std::array<int, 10> key = tiling_key(s);
     {
         std::lock_guard<std::mutex> lk(g_tilings_mu);
         auto it = g_tilings.find(key);
@@ -395,13 +413,24 @@ int start_tuning(armon_solver* s)
     // resident blocks per axis
     const int halo = stencil_reach(&p);
     const int block = s->o.block_lines > 0 ? s->o.block_lines : 128;
-    std::vector<int> forms;
+    std::vector<int> forms, waves;
     auto& T = s->tune;
     if (s->tile) {
-        // columns of a Y tile: the usual number and four
-        for (int lines : {s->fp32 ? tile_y_lines<float>() : tile_y_lines<double>(), 4})
-            T.cand.push_back(Tiling{0, lines, block, kTileForm});
-    } else if (s->d_faces && s->o.split_pass == 0) forms = {1, 0}; else forms = {s->split ? 1 : 0};
+        const int lines = s->fp32 ? tile_y_lines<float>() : tile_y_lines<double>();
+        T.cand.push_back(Tiling{0, lines, block, kTileForm});
+        if (s->fp32 && s->o.reuse >= 0 && (int64_t)p.nx * p.ny < (1 << 23)) {
+            T.cand.push_back(Tiling{scan_default<float>(p) ? -1 : 1, lines, block, kTileForm});
+        } else {
+            T.cand.push_back(Tiling{0, 4, block, kTileForm});   // columns of a Y tile
+        }
+    } else {
+        if (s->d_faces && s->o.split_pass == 0) forms = {1, 0}; else forms = {s->split ? 1 : 0};
+        // FP32 also tries shorter segments (12 and 16 waves): 96-cell segments ran the 8192² run 3 %
+        // faster than 144 throughout, whereas FP64's 36-cell segments, which win the cycles the
+        // measurement runs on (thin fronts), lost 9 % on the late cycles of the 4096² run
+        waves = {1, 2, 3, 4, 6, 8};
+        if (s->fp32) waves.insert(waves.end(), {12, 16});
+    }
     for (int form : forms) {
         const int per_sm = form ? sweep_split_blocks_per_sm(s->fp32, p.scheme, p.projection, block)
                                 : sweep_blocks_per_sm(s->fp32, p.scheme, p.projection, block);
@@ -412,11 +441,7 @@ int start_tuning(armon_solver* s)
             model[axis] = choose_segments(n, nl, block, halo, s->sm_count, 0).seg_len;
         }
         T.cand.push_back(model);
-        // FP32 also tries shorter segments (12 and 16 waves): 96-cell segments ran the 8192² run 3 %
-        // faster than 144 throughout, whereas FP64's 36-cell segments, which win the cycles the
-        // measurement runs on (thin fronts), lost 9 % on the late cycles of the 4096² run
-        for (int w : {1, 2, 3, 4, 6, 8, 12, 16}) {
-            if (w > 8 && !s->fp32) continue;
+        for (int w : waves) {
             Tiling c{0, 0, block, form};
             for (int axis = 0; axis < 2; axis++) {
                 const int n = axis == 0 ? p.nx : p.ny, nl = axis == 0 ? p.ny : p.nx;
@@ -487,10 +512,10 @@ int finish_tuning(armon_solver* s)
         if (visits[i] < 2) continue;
         if (!have || total[i] < best_t) { best = i; best_t = total[i]; have = true; }
     }
-    // tiles: the usual columns unless the others win by more than two timed cycles differ
+    // tiles: the usual ones unless the others win by more than two timed cycles differ
     if (have && T.cand[0][3] == kTileForm && visits[0] >= 2 && total[0] < 1.03f * best_t) best = 0;
     const Tiling choice = ran && have ? T.cand[best] : model_tiling(s);
-    const std::array<int, 9> key = T.key;
+    const std::array<int, 10> key = T.key;
     end_tuning(s);
     s->tuned = ran;
     rc = apply_tiling(s, choice);
@@ -764,6 +789,7 @@ int armon_solver_init_test(armon_solver* s)
                  s->arr[6], s->arr[7], s->arr[8], s->arr[9], s->arr[10]};
     CUDA_TRY(launch_init(a, p.nb_cells, ptr, s->fp32, s->stream));
     s->launches++;
+    s->from_test = true;
     return armon_solver_begin_loop(s);
 }
 

@@ -92,8 +92,9 @@ template <class T> constexpr int tile_y_lines() { return sizeof(T) == 8 ? 2 : 8;
 // in FP32 (8 and 16 cost its streamed domains 2-5 %), 8 in FP64 (1001x573 Godunov 7.6 ms, against 9.0
 // with 4; the moving flow and the circular Sod within 1 %), 16 in an FP64 batch, whose domains end one
 // by one (16 uneven domains 159 ms, against 172 with 8, 179 with 4, 166 with 32).
+// scan: units may be scanned for uniform regions, where there are enough of them.
 template <class T>
-void set_tile_axis(AxisGeom<T>& g, bool rows, int halo, int sms, int slots, int y_lines, int tail)
+void set_tile_axis(AxisGeom<T>& g, bool rows, int halo, int sms, int slots, int y_lines, int tail, bool scan)
 {
     const int want = rows ? 1 : std::max(1, std::min(y_lines, g.nlines));
     const int longest = std::max(1, rows ? std::min(248, kTileBlock - 2 * halo) : kTileBlock / want / 8 * 8 - 2 * halo);
@@ -109,7 +110,7 @@ void set_tile_axis(AxisGeom<T>& g, bool rows, int halo, int sms, int slots, int 
     g.tile_groups = (g.nlines + g.tile_lines - 1) / g.tile_lines;
     // worth a scan when a block has several tiles; the walls' positions may not overlap, and a stretch's
     // first position is held in 23 bits
-    g.tile_scan = (rows ? g.tile_lines == 1 : g.tile_lines * kTileUnit <= 64 && (g.tile_width + 7) / 8 * 8 * g.tile_lines <= kTileBlock) && g.n >= 32 &&
+    g.tile_scan = scan && (rows ? g.tile_lines == 1 : g.tile_lines * kTileUnit <= 64 && (g.tile_width + 7) / 8 * 8 * g.tile_lines <= kTileBlock) && g.n >= 32 &&
                   g.n < (1 << 23) &&
                   (int64_t)segs * g.tile_groups >= 3 * (int64_t)slots;
     if (!rows && g.tile_scan)       // a large unit of columns lies in one segment
@@ -118,6 +119,17 @@ void set_tile_axis(AxisGeom<T>& g, bool rows, int halo, int sms, int slots, int 
     int64_t big = std::max<int64_t>(0, (tiles - tail * (int64_t)slots) / kTileUnit);
     g.tile_big = (int)big;
     g.tile_units = (int)(big + (tiles - big * kTileUnit));
+}
+
+// Whether a lone domain's units are scanned before any measurement.  FP64 domains are wherever they have
+// the units: 640x640 circular Sod, 60 cycles, 9.9 ms scanned and 11.8 computed, 512x512 8.5 and 8.3.  An
+// FP32 position costs a tenth, while a unit whose eight tiles are all computed keeps its block ~0.1 ms:
+// scanned, 60 cycles take 15 to 20 ms from 640x640 to 2048x2048; computed 3.3 ms at 640x640, 5.5 at
+// 1024x1024, 11.4 at 1536x1536, 17.0 at 2048x2048, 23.8 at 2304x2304 (16.4 scanned), and 8192x500 17.7
+// (18.2), 4096x1200 21.0 (16.4).  (A batch shares its blocks out by cells and scans in both.)
+template <class T> inline bool scan_default(const armon_params& p)
+{
+    return sizeof(T) == 8 || (int64_t)p.nx * p.ny >= 4500000;
 }
 
 inline int check_supported(const armon_params* p)

@@ -167,7 +167,8 @@ int64_t armon_solver_kernel_launches(armon_solver* s);
  * axis and blocks per launch.  Unless opts.seg_len fixes it, a domain of 2^20 cells or more gets the fastest of a few
  * candidate tilings, each timed on real cycles of its first time loop (after 16 cycles with the
  * model's tiling, two cycles per candidate forwards and two backwards: results never depend on
- * the tiling), and cached per geometry for the process; smaller domains use the cost model. */
+ * the tiling), and cached for the process per geometry and per what the loop starts from (a test
+ * problem of init_test, or the caller's own state); smaller domains use the cost model. */
 int armon_solver_tiling(armon_solver* s, int32_t seg_len[2], int32_t blocks[2]);
 /* Lines (threads) per block of a march: the caller's block_lines, or the measured choice. */
 int armon_solver_block_lines(const armon_solver* s);
@@ -180,8 +181,8 @@ int64_t armon_solver_measurement_cycles(const armon_solver* s);
 /* 1 when the axis passes run split (a face launch and a cell launch), 0 when a pass is one launch
  * (tiles, or fused marches). */
 int armon_solver_split_pass(const armon_solver* s);
-/* Forgets the tilings measured so far in this process (the next time loop of each geometry
- * measures again). */
+/* Forgets the tilings measured so far in this process (the next time loop of each geometry measures
+ * again). */
 void armon_tiling_cache_clear(void);
 
 /* ---- batches: many independent domains advanced together (no counterpart in the reference;

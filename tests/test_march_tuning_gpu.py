@@ -68,3 +68,42 @@ def test_march_batches_choose_their_waves_and_keep_the_results(precision, split_
     assert seen[:5] == [2, 4, 8, 16, 64] and seen[5] == seen[6] == seen[7] and seen[5] in seen[:5]
     for a, c in zip(*out):
         same(a, c)
+
+
+@pytest.mark.parametrize("precision", [64, 32])
+def test_a_measured_choice_belongs_to_what_the_loop_starts_from(precision):
+    # one test problem's choice is not another's, nor that of a state that the caller uploads, for a new solver
+    # as for the same one
+    kw = dict(scheme="GAD", projection="euler_2nd", nghost=5, nx=1024, ny=1056, cfl=0.6, max_cycles=40, max_time=1e9)
+    sod, sedov = (A.Case(test=t, **kw) for t in ("Sod", "Sedov"))
+    A.tiling_cache_clear()
+    with A.Solver(sod, precision=precision) as s:
+        s.init_test()
+        assert s.tuning()
+        s.run()
+        assert s.measurement_cycles() > 0
+        s.init_test()
+        assert not s.tuning()
+        state = {k: s.download(k) for k in ("rho", "umat", "vmat", "Emat")}
+        for k, a in state.items():
+            s.upload(k, a)
+        s.begin_loop()
+        assert s.tuning()
+        s.run()
+        own = fields(s)
+        s.init_test()
+        assert not s.tuning()
+        s.run()
+        same(fields(s), own)
+    with A.Solver(sedov, precision=precision) as s:
+        s.init_test()
+        assert s.tuning()
+        s.run(cycle_limit=21)             # a candidate is in use
+        s.init_test()
+        s.run()
+        again = fields(s)
+    with A.Solver(sedov, precision=precision, reuse=-1) as s:
+        s.init_test()
+        s.run()
+        same(fields(s), again)
+    A.tiling_cache_clear()

@@ -12,9 +12,9 @@ from test_tile_gpu import patches, same, solve
 TILE = ("len", "width", "lines", "segs", "groups", "scan", "big", "units")
 
 
-def tile_axis(n, nlines, rows, halo, slots, y_lines, tail):
+def tile_axis(n, nlines, rows, halo, slots, y_lines, tail, scan=True):
     out = (C.c_int32 * 8)()
-    A.lib().armon_selftest_tile_axis(n, nlines, int(rows), halo, 152, slots, y_lines, tail, out)
+    A.lib().armon_selftest_tile_axis(n, nlines, int(rows), halo, 152, slots, y_lines, tail, int(scan), out)
     return dict(zip(TILE, out))
 
 
@@ -56,6 +56,7 @@ def test_tiles_cover_each_cell_once_and_fit_the_block(halo, y_lines, tail):
                     assert (g["segs"] - 1) * g["len"] < n <= g["segs"] * g["len"]
                     assert (g["groups"] * g["lines"] >= nlines) and g["lines"] <= nlines
                     tiles = g["segs"] * g["groups"]
+                    assert not tile_axis(n, nlines, rows, halo, slots, y_lines, tail, scan=False)["scan"]
                     assert g["units"] == g["big"] + tiles - 8 * g["big"] and 0 <= 8 * g["big"] <= tiles
                     if g["scan"]:
                         assert n >= 32 and tiles >= 3 * slots
@@ -73,10 +74,10 @@ def test_tiles_cover_each_cell_once_and_fit_the_block(halo, y_lines, tail):
 # scanned domains whose last segment along Y (FP32: eight columns a tile, FP64: two) or X is shorter than a
 # stretch of eight threads: reach 2 (Godunov, euler) with up to three cells, reach 3 with one
 SHORT = [
-    ("Godunov", "euler", 32, 811, 757, 1, 1), ("Godunov", "euler", 32, 811, 731, 1, 3),
-    ("GAD", "euler", 32, 811, 651, 1, 1), ("Godunov", "euler_2nd", 32, 811, 677, 1, 1),
+    ("Godunov", "euler", 32, 6011, 757, 1, 1), ("Godunov", "euler", 32, 6211, 731, 1, 3),
+    ("GAD", "euler", 32, 7011, 651, 1, 1), ("Godunov", "euler_2nd", 32, 6711, 677, 1, 1),
     ("Godunov", "euler", 64, 48, 15007, 1, 3), ("GAD", "euler", 64, 48, 14763, 1, 1),
-    ("Godunov", "euler", 64, 60763, 16, 0, 3), ("Godunov", "euler", 32, 60763, 16, 0, 3),
+    ("Godunov", "euler", 64, 60763, 16, 0, 3), ("Godunov", "euler", 32, 60763, 80, 0, 3),
 ]
 
 
@@ -86,6 +87,7 @@ def test_short_last_segments_are_what_the_solves_below_scan(scheme, projection, 
     n, lines = (ny, nx) if axis else (nx, ny)
     g = tile_axis(n, lines, axis == 0, halo, 152 * (3 if precision == 64 else 4), 2 if precision == 64 else 8,
                   8 if precision == 64 else 4)
+    assert A.lib().armon_selftest_scan_default(nx, ny, precision)
     assert g["scan"] and n - (g["segs"] - 1) * g["len"] == last
 
 
