@@ -303,7 +303,9 @@ int ensure_stage(armon_solver* s)
 // Tiling of a lone domain, measured on the caller's own cycles.  The tile form compares two widths of
 // its Y tiles, or, in FP32 below 2^23 cells, units scanned and not: which is faster there depends on how
 // much of the domain is at rest (2048x2048, 60 cycles: circular Sod 22 ms scanned and 17.0 computed, Sedov
-// 8.4 and 17).
+// 8.4 and 17).  A planar test problem (planar_test) adds fused marches in segments of 48 and 16 (FP32: 24)
+// cells, short enough for the front's own positions later in the run: planar Sod at 1024x1024, 500 cycles,
+// 116 ms in FP64 against 181 in tiles, 42 in FP32 against 46.
 // For marches with the GPU to itself, the best segment length depends on more than the cells a thread
 // walks (how full the last wave of blocks is, how many blocks share an SM, how unevenly the units cost
 // -- fronts against fluid at rest --, cache traffic), and so does the pass form (split passes keep the
@@ -384,6 +386,13 @@ void end_tuning(armon_solver* s)
     s->tune = armon_solver::Tune{};
 }
 
+// Whether the loop started from a planar test problem: all lines along the front hold one state each, for
+// the whole run, and marches stream such lines whatever the states are, where a scan knows two of them.
+bool planar_test(const armon_solver* s)
+{
+    return s->o.reuse >= 0 && (s->source == 1 + ARMON_SOD || s->source == 1 + ARMON_SOD_Y);
+}
+
 // Called by begin_loop: the cached tiling of this geometry, or the measurement's set-up.
 int start_tuning(armon_solver* s)
 {
@@ -423,6 +432,8 @@ int start_tuning(armon_solver* s)
         } else {
             T.cand.push_back(Tiling{0, 4, block, kTileForm});   // columns of a Y tile
         }
+        if (planar_test(s))
+            for (int seg : {s->fp32 ? 24 : 16, 48}) T.cand.push_back(Tiling{seg, seg, block, 0});
     } else {
         if (s->d_faces && s->o.split_pass == 0) forms = {1, 0}; else forms = {s->split ? 1 : 0};
         // FP32 also tries shorter segments (12 and 16 waves): 96-cell segments ran the 8192² run 3 %

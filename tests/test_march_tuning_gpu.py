@@ -107,3 +107,27 @@ def test_a_measured_choice_belongs_to_what_the_loop_starts_from(precision):
         s.run()
         same(fields(s), again)
     A.tiling_cache_clear()
+
+
+@pytest.mark.parametrize("precision", [64, 32])
+@pytest.mark.parametrize("test", ["Sod", "Sod_y", "Sod_circ", "Sedov"])
+@pytest.mark.parametrize("shape", [(1024, 1056), (2400, 1900), (700, 6600)])
+def test_candidates_of_every_form_keep_the_results(shape, test, precision):
+    # tiles scanned and computed, and marches for planar fronts, one after another on the cycles of one solve
+    nx, ny = shape
+    case = A.Case(test=test, scheme="GAD", projection="euler_2nd", nghost=5, nx=nx, ny=ny, cfl=0.5, max_cycles=40,
+                  max_time=1e9)
+    A.tiling_cache_clear()
+    out = []
+    for kw in (dict(), dict(), dict(reuse=-1), dict(split_pass=-1, seg_len=64)):
+        with A.Solver(case, precision=precision, **kw) as s:
+            s.init_test()
+            s.run()
+            p, status = s.state()
+            assert status == 0 and p.cycle == 40 and not s.tuning()
+            assert kw or len(out) or s.measurement_cycles() == (16 if test in ("Sod", "Sod_y") else 8)
+            out.append((fields(s), (p.time, p.current_cycle_dt, p.next_cycle_dt)))
+    for got, end in out[1:]:
+        assert end == out[0][1]
+        same(got, out[0][0])
+    A.tiling_cache_clear()
