@@ -56,6 +56,7 @@ struct Dom {
     void* faces = nullptr;        // split passes: 3 face arrays of face_values(p) values
     int seg_len = 0;
     bool eos_stale = false;       // tile passes have run since p, c, g were stored
+    bool planar = false;          // started from a planar front along one axis
 };
 
 // values per face array of a split pass (sweep_split.cuh): the larger axis's (n + 5) * nlines
@@ -110,7 +111,7 @@ struct armon_batch {
     cudaGraphExec_t graph = nullptr;
     int64_t bytes = 0;
     int64_t launches = 0;
-    bool tile = true;             // passes in the tile form (sweep_tile.cuh), unless a domain fixes its segments
+    bool tile = true;             // passes may run in the tile form (sweep_tile.cuh): wants_tiles
     bool tiled = true;            // the current table's form
     int* d_units = nullptr;       // tile form: units of each domain
     int* d_rest = nullptr;        // the domains that no block starts on
@@ -269,6 +270,28 @@ int rebuild_tiles(armon_batch* b)
     return ARMON_OK;
 }
 
+// Whether the running domains' passes run in tiles.  Marches take domains that a caller gives segments to,
+// and many planar domains: a planar front's lines along it hold one state each, whatever it is, which
+// marches stream, while a scan knows two states.  (Sod to the reference's walls, ms FP64 / FP32 in tiles
+// and in marches: 200 of 128x128, 100 cycles, 152 / 41 and 91 / 26; 16 of 256x256, 200 cycles, 104 / 32 and
+// 63 / 19; 8 of 256x256 59 / 26 and 44 / 15; 16 of 512x512 190 / 61 and 141 / 48.  With fewer cells a pass of
+// marches is one segment's positions: 16 of 100x100, 100 cycles, 11 / 5 and 26 / 7.  Larger domains have
+// more at rest: 4 of 1024x1024 150 / 53 and 150 / 46 along X, 125 / 41 and 167 / 49 along Y; 3 of 2048x1500
+// 178 / 76 and 300 / 92.)
+bool wants_tiles(const armon_batch* b)
+{
+    if (!b->tile) return false;
+    bool planar = b->o.reuse >= 0;
+    int64_t cells = 0;
+    for (int i : b->table) {
+        const Dom& d = b->doms[i];
+        if (d.seg_len > 0) return false;
+        planar = planar && d.planar;
+        cells += (int64_t)d.p.nx * d.p.ny;
+    }
+    return !planar || cells < (1 << 19) || cells >= 400000 * (int64_t)b->table.size();
+}
+
 // The launch table of the running domains.  The batch stays dirty until it is complete: a rebuild that
 // fails is made again before anything is launched.
 template <class T>
@@ -278,8 +301,7 @@ int rebuild_t(armon_batch* b)
     b->table.clear();
     for (int i = 0; i < (int)b->doms.size(); i++)
         if (b->doms[i].used && !b->doms[i].done) b->table.push_back(i);
-    bool tiled = b->tile;
-    for (int i : b->table) tiled = tiled && b->doms[i].seg_len <= 0;
+    const bool tiled = wants_tiles(b);
     if (tiled != b->tiled) b->blocks_per_sm = 0;
     b->tiled = tiled;
     if (tiled && b->tune.phase == 1) {
@@ -656,6 +678,8 @@ int add_domain(armon_batch* b, const armon_params* p, const double* const init[4
     Dom d;
     d.p = *p;
     d.bytes = need;
+    d.planar = sod ? sod->shape == 0 && (sod->nx == 0 || sod->ny == 0)
+                   : !init && (p->test == ARMON_SOD || p->test == ARMON_SOD_Y);
     cudaError_t e = cudaMallocFromPoolAsync(&d.chunk, (size_t)need, b->pool, b->stream);
     if (e != cudaSuccess) return cuda_fail(e, "cudaMallocFromPoolAsync");
     char* base = (char*)d.chunk;

@@ -193,7 +193,8 @@ typedef struct armon_batch_opts {
     int32_t precision;        /* 64 or 32: every domain of a batch has this precision */
     int32_t cycles_per_graph; /* cycles captured per CUDA graph launch (default 8) */
     /* block_lines 128, seg_len, waves and split_pass 0 (default): passes in the tile form, as a
-       solver's.  Anything else selects the marches. */
+       solver's, or in marches while armon_batch_set_seg_len asks for segments or all running domains
+       are many planar ones (results never depend on the form).  Anything else selects the marches. */
     int32_t block_lines;      /* marches: lines (threads) per block: a multiple of 32, at most 128 (default 128) */
     int32_t seg_len;          /* marches: cells per thread along the sweep axis for every domain (0 = scheduled) */
     int64_t memory_budget;    /* bytes of domain state the batch may hold (0 = no limit) */

@@ -135,3 +135,60 @@ def test_many_small_domains_and_a_large_one_match_solo(precision):
             for f in FIELDS if n % 20 < 4 or k == 4 else ("rho",):
                 got = A.real_cells(b.params[i], b.download(i, f))
                 assert np.array_equal(got.view(np.int64), refs[k][1][f].view(np.int64)), (n, f)
+
+
+@pytest.mark.parametrize("precision", [64, 32])
+def test_planar_domains_run_in_marches_while_they_are_many(precision):
+    # 40 planar domains, most of which end early: marches until fewer than 2^19 cells are left, tiles after
+    # that and whenever a front that is not planar is among them
+    def case(test, cycles):
+        return A.Case(test=test, scheme="GAD", projection="euler_2nd", nghost=5, nx=128, ny=144, cfl=0.6, max_cycles=cycles,
+                      max_time=1e9)
+
+    kinds = [case("Sod", 8), case("Sod_y", 8), case("Sod", 20), case("Sod_circ", 12)]
+    refs = []
+    for c in kinds:
+        with A.Solver(c, precision=precision) as s:
+            s.init_test()
+            s.run()
+            p, _ = s.state()
+            refs.append(((p.cycle, p.time, p.next_cycle_dt), {k: A.real_cells(s.params, s.download(k)) for k in FIELDS}))
+    per_cycle = {True: 2, False: 5 if precision == 64 else 3}     # launches: tiles; marches and their block order
+    for circular in (False, True):
+        with A.Batch(precision=precision, cycles_per_graph=4) as b:
+            order = [0, 1] * 17 + [2] * 6 + [3] * circular
+            ids = [b.add(A.make_params(kinds[k])) for k in order]
+            b.run(cycle_limit=4)
+            for tiles in (circular, True):
+                before = b.kernel_launches
+                b.run(cycle_limit=4)
+                # (a new table of marches starts from index order: one launch more)
+                assert 0 <= b.kernel_launches - before - 4 * per_cycle[tiles] <= 1
+            assert b.run() == 0
+            for i, k in zip(ids, order):
+                p, st = b.state(i)
+                assert st == 0 and (p.cycle, p.time, p.next_cycle_dt) == refs[k][0]
+                for f in FIELDS:
+                    got = A.real_cells(b.params[i], b.download(i, f))
+                    assert np.array_equal(got.view(np.int64), refs[k][1][f].view(np.int64)), (k, f)
+
+
+def test_interfaces_along_an_axis_count_as_planar():
+    def launches(shape, nx, ny):
+        c = A.Case(test="Sod", scheme="GAD", projection="euler_2nd", nghost=5, nx=256, ny=256, cfl=0.6, max_cycles=8, max_time=1e9)
+        sod = A.SodInterface(shape=shape, cx=0.5, cy=0.5, nx=nx, ny=ny, offset=0.0, r2=0.04, rho_high=1.0, p_high=1.0,
+                             rho_low=0.125, p_low=0.1)
+        with A.Batch(cycles_per_graph=4) as b:
+            ids = [b.add_sod(c, sod) for _ in range(8)]
+            b.run(cycle_limit=4)
+            before = b.kernel_launches
+            b.run(cycle_limit=4)
+            n = b.kernel_launches - before
+            return n, [b.download(i, "rho") for i in ids]
+
+    for nx, ny in ((1.0, 0.0), (0.0, 1.0)):
+        n, rho = launches(0, nx, ny)
+        assert n == 4 * 5 and all(np.array_equal(rho[0], r) for r in rho)
+    for shape, nx, ny in ((0, 0.6, 0.8), (1, 0.0, 0.0)):
+        n, rho = launches(shape, nx, ny)
+        assert n == 4 * 2 and all(np.array_equal(rho[0], r) for r in rho)
