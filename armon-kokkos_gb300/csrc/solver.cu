@@ -786,12 +786,7 @@ int armon_solver_begin_loop(armon_solver* s)
 
 int armon_solver_init_test(armon_solver* s)
 {
-    if (s->begun) {
-        // the arrays hold the current state before they are written: begin_loop would put it back over them
-        int rc = sync_state(s);
-        if (rc == ARMON_OK) rc = settle(s);
-        if (rc != ARMON_OK) return rc;
-    }
+    s->begun = false;      // no earlier state for begin_loop to put back over the arrays
     const armon_params& p = s->p;
     InitArgs a{};
     a.row_length = p.row_length; a.nb_ghosts = p.nb_ghosts; a.nx = p.nx; a.ny = p.ny;
