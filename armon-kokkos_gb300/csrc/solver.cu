@@ -2,9 +2,9 @@
 // (include/armon_gb300.h).
 //
 // One cycle = passes_per_cycle(splitting) axis passes, each one launch in the tile form
-// (sweep_tile.cuh), or a march when the caller's options ask for one: one fused launch, or a face and a
-// cell launch.  The last one also reduces dt_CFL of the new
-// state and commits the cycle (time, cycle, dts) into the device StepState, so the host never
+// (sweep_tile.cuh), or a march (one fused launch, or a face and a cell launch) when the caller's options
+// ask for one or a planar problem's measurement finds it faster.  The last one also reduces dt_CFL of the
+// new state and commits the cycle (time, cycle, dts) into the device StepState, so the host never
 // waits inside the loop.  Cycles are issued in batches captured in a CUDA graph;
 // after each batch the host reads the 64-byte state back to test the reference's loop condition
 // (time < max_time && cycle < max_cycles).  Cycles issued past the end are no-ops on the device.

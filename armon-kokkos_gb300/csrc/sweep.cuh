@@ -37,8 +37,9 @@
 //
 // This file holds the stage functions, the fused march and its batch kernel; sweep_split.cuh marches
 // the same stages as two launches per pass, and order.cuh orders each launch's units longest first.
-// The marches run when a caller fixes segments, block lines, waves or the pass form; otherwise passes
-// run the same stages in tiles (sweep_tile.cuh).
+// The marches run when a caller fixes segments, block lines, waves or the pass form, and for planar
+// test problems (solver.cu planar_test, batch.cu wants_tiles); otherwise passes run the same stages in
+// tiles (sweep_tile.cuh).
 #pragma once
 
 #include "device_common.cuh"
@@ -200,7 +201,7 @@ struct AxisGeom {
     int32_t tile_groups;  // tiles across the lines
     int32_t tile_units;   // units of the axis: tile_big of kTileUnit consecutive tiles, then one tile each
     int32_t tile_big;
-    int32_t tile_scan;    // units may be scanned for kept states (one row, or up to 32 columns, per unit)
+    int32_t tile_scan;    // units may be scanned for kept states (eight rows' tiles, or up to 64 columns, per unit)
 };
 
 // States that uniform regions of a domain probably hold (sweep_tile.cuh), per state buffer set:

@@ -16,8 +16,12 @@
 // busy in each of two launches): 0.94 ms an X pass; 24 cycles 78.2 ms with marches, 45.9 ms now.  FP32
 // there: instruction issue, 70 % busy, 0.14 ms.  A uniform fluid with fronts (4096x4096 circular Sod):
 // a block's own chain of scan, stores and computed stretches (30 000 cycles each), three blocks per
-// SM; 0.38-0.45 ms a pass late in the run, against 1.1 ms.  Small domains: one position's ~3000
-// dependent instructions, 16 us a pass (96x64: 42 us a cycle, 546 us with marches).
+// SM; 0.55 ms a pass at cycles 180-200, against 1.1 ms.  Small domains: one position's ~3000
+// dependent instructions, 16 us a pass (96x64: 40 us a cycle, 546 us with marches).
+// Where it loses to marches: planar fronts.  Every line along one holds a state of its own, which a march
+// streams; a scan knows two states and computes the rest (solver.cu planar_test, batch.cu wants_tiles).
+// Looking for runs of any state in units that are not all idle made planar fronts 1.3 to 1.6 times
+// faster in FP64 and the 4096x4096 circular Sod 20 to 30 % slower (code size), and was dropped.
 // Measured and dropped: 64 registers and four blocks per SM in FP64 (spills; +4 to +20 %), products on
 // the integer pipes (dense 5 % faster at best, fronts 15-40 % slower), the quotients of a stage in one
 // straight-line group (+7 to +10 %: more code), cells of the next unit asked for in L2 (+8 %),
@@ -667,7 +671,9 @@ struct TilePass {
 
     // The stages at the thread's position; ds threads between neighbouring positions.  The centre
     // thread records its state when it can.  Returns sh.claims as every thread of the block sees it: read
-    // between the barrier that follows this call's claim and the ones before the next call's.
+    // between the barrier that follows this call's claim and the ones before the next call's.  (Nothing
+    // else that a claim writes, sh.turn and sh.kept among it, may decide a branch between two calls: the
+    // centre's warp may be in the next one already, and warps that disagree meet different barriers.)
     __device__ __forceinline__ int compute(const AxisGeom<T>& g, const Spot& p, const int ds, const int centre)
     {
         const int tid = threadIdx.x;

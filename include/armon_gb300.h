@@ -84,8 +84,9 @@ typedef struct armon_solver_opts {
                                  32: FP32 state and arithmetic, FP64 dt and conservation sums */
     int32_t cycles_per_graph; /* cycles captured per CUDA graph launch (0 = default, 16) */
     /* seg_len, block_lines and split_pass all 0 (default): the axis passes run in the tile form, one
-       thread per position (csrc/sweep_tile.cuh).  Any of them set selects the marches, one thread per
-       line segment.  Results are the same bits in every form. */
+       thread per position (csrc/sweep_tile.cuh); only a planar test problem's tiling measurement may
+       choose fused marches.  Any of them set selects the marches, one thread per line segment.  Results
+       are the same bits in every form. */
     int32_t seg_len;          /* marches: cells per thread along the sweep axis (0 = automatic) */
     int32_t block_lines;      /* marches: lines (threads) per block (0 = automatic, 128) */
     int32_t materialize_eos;  /* p, c, g of the real cells: written by every pass (1), by the last
