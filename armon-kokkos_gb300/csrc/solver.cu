@@ -344,10 +344,12 @@ int refill(armon_solver* s)
 int ensure_partials(armon_solver* s)
 {
     if (s->grid <= s->partials_cap) return ARMON_OK;
+    // (the old buffer stays in use when there is no room for a larger one)
+    double* larger = nullptr;
+    CUDA_TRY(cudaMalloc(&larger, sizeof(double) * 2 * (size_t)s->grid));
     CUDA_TRY(cudaStreamSynchronize(s->stream));
     CUDA_TRY(cudaFree(s->d_partials));
-    s->d_partials = nullptr;
-    CUDA_TRY(cudaMalloc(&s->d_partials, sizeof(double) * 2 * (size_t)s->grid));
+    s->d_partials = larger;
     s->partials_cap = s->grid;
     if (s->fp32) s->a32.partials = s->d_partials; else s->a64.partials = s->d_partials;
     return ARMON_OK;
@@ -415,7 +417,9 @@ int start_tuning(armon_solver* s)
         auto it = g_tilings.find(key);
         if (it != g_tilings.end()) {
             s->tuned = true;
-            return apply_tiling(s, it->second);
+            if (apply_tiling(s, it->second) == ARMON_OK) return ARMON_OK;
+            cudaGetLastError();         // no room for it here
+            return apply_tiling(s, model_tiling(s));
         }
     }
     // candidates per form and block size: the model's tiling, then segments aiming at w waves of
@@ -555,7 +559,14 @@ int enqueue(armon_solver* s, int n_cycles)
         } else if (T.warm) {
             // the candidate's first cycle records its units' costs for longest-first dispatch
             rc = apply_tiling(s, T.cand[T.seq[T.pos]]);
-            if (rc == ARMON_OK) rc = enqueue_direct(s, 1);
+            if (rc != ARMON_OK) {       // no room for its block order or partials: the usual tiling, nothing cached
+                cudaGetLastError();
+                end_tuning(s);
+                rc = apply_tiling(s, model_tiling(s));
+                if (rc != ARMON_OK) return rc;
+                break;
+            }
+            rc = enqueue_direct(s, 1);
             T.warm = false;
             s->measure_cycles++;
         } else {
